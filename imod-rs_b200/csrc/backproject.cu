@@ -32,42 +32,10 @@
 #include "tg_internal.h"
 #include "f32x2.cuh"
 #include "local_dev.cuh"
+#include "pipe.cuh"
 
 namespace tg {
 
-__device__ __forceinline__ uint32_t smem_u32(const void *p) {
-  return (uint32_t)__cvta_generic_to_shared(p);
-}
-__device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
-}
-__device__ __forceinline__ void fence_mbar_init() {
-  asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-}
-__device__ __forceinline__ void fence_proxy_async() {
-  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-}
-__device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes)
-               : "memory");
-}
-__device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-      " selp.u32 %0, 1, 0, p;\n}\n"
-      : "=r"(ok)
-      : "r"(bar), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-__device__ __forceinline__ void bulk_g2s(uint32_t dst, const void *src, uint32_t bytes,
-                                         uint32_t bar) {
-  asm volatile(
-      "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
-      "l"(src), "r"(bytes), "r"(bar)
-      : "memory");
-}
 __device__ __forceinline__ float4 lds128(uint32_t a) {
   float4 v;
   asm volatile("ld.shared.v4.f32 {%0,%1,%2,%3}, [%4];"
@@ -128,9 +96,6 @@ template <int I, int N, class F> __device__ __forceinline__ void static_for(F &&
   }
 }
 
-constexpr float MAGIC = 12582912.0f;      // 1.5 * 2^23
-constexpr uint32_t MAGIC_BITS = 0x4B400000u;
-
 // exact reference position for (dx, dz): ((dx*c)*cxt + (dz*s)*zf) + cx.
 // ZF: 0 no z-factor, 1 z-factor, 2 z-factor and x-tilt (t1 carries *cos_xt)
 template <int ZF>
@@ -155,42 +120,9 @@ struct FastCfg {
   static size_t smem(int nviews) { return BUF + 8 * (size_t)nviews + 16 * NSTAGE + 16 + 64; }
 };
 
-__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
-}
 __device__ __forceinline__ void consumer_sync(int nthreads) {
   asm volatile("bar.sync 1, %0;" ::"r"(nthreads) : "memory");
 }
-// try_wait that lets the hardware suspend the thread (up to hint_ns) until the
-// phase completes, instead of returning at once
-__device__ __forceinline__ bool mbar_try_wait_sleep(uint32_t bar, uint32_t parity, uint32_t hint_ns) {
-  uint32_t ok;
-  asm volatile(
-      "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n"
-      " selp.u32 %0, 1, 0, p;\n}\n"
-      : "=r"(ok)
-      : "r"(bar), "r"(parity), "r"(hint_ns)
-      : "memory");
-  return ok != 0;
-}
-__device__ __forceinline__ uint64_t globaltimer_ns() {
-  uint64_t t;
-  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-  return t;
-}
-// Bounded wait on an mbarrier phase: sleeps in try_wait, gives up after limit_ns
-// of wall time (BpArgs::wait_limit_ns, 2 s by default: a stage never
-// legitimately takes that long) or, when abort is given, as soon as another warp
-// of the CTA has given up.
-__device__ __forceinline__ bool wait_phase(uint32_t bar, uint32_t parity, volatile int *abort, uint64_t limit_ns) {
-  if (mbar_try_wait(bar, parity)) return true;
-  const uint64_t t0 = globaltimer_ns();
-  for (;;) {
-    if (mbar_try_wait_sleep(bar, parity, 20000u)) return true;
-    if ((abort && *abort) || globaltimer_ns() - t0 > limit_ns) return false;
-  }
-}
-
 // Warp-specialised pipeline: warp NT/32 (the producer) copies each stage's
 // per-view row windows with cp.async.bulk, one copy per lane, completing on
 // full[b]; consumer warps wait on full[b], accumulate, and release the buffer

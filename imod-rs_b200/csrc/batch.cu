@@ -18,17 +18,30 @@ using namespace tg;
 
 namespace tg {
 
-// One persistent launch per (storage, z-factor, tile variant) group of fast-path
-// series, each series keeping the tile shape tuned for it; other series get
+long long bp_group_tiles(const BpGroup &g, BpArgs &a) {
+  if (std::get<2>(g) < 0) return bp_mma_plan(a);
+  int S, TX, TZ;
+  bp_fast_tile_shape(std::get<2>(g), &S, &TX, &TZ);
+  a.nbx = (a.onx + TX - 1) / TX;
+  a.ntiles_xz = a.nbx * ((a.onz + TZ - 1) / TZ);
+  return (long long)a.ntiles_xz * ((a.ny + S - 1) / S);
+}
+
+int launch_bp_group(const BpGroup &g, const BatchLaunch &bl, cudaStream_t st) {
+  if (std::get<2>(g) < 0) return launch_bp_mma_batch(bl, std::get<1>(g), st);
+  return launch_bp_batch(bl, std::get<0>(g), std::get<1>(g) != 0, std::get<2>(g), st);
+}
+
+// One launch per group (bp_group) of fast-path series; other series get
 // their own launch.  ntiles[i] receives the partial-stat
 // tile count written for ss[i] (used when modes[i] == 0).
 int batch_bp(tg_batch *b, const std::vector<tg_session *> &ss, const std::vector<int> &modes,
              std::vector<int> &ntiles, int *launches) {
   ntiles.assign(ss.size(), 0);
-  std::map<std::tuple<int, int, int>, std::vector<int>> groups;
+  std::map<BpGroup, std::vector<int>> groups;
   for (size_t i = 0; i < ss.size(); ++i) {
     if (ss[i]->fast)
-      groups[std::make_tuple(ss[i]->store, ss[i]->zf_any ? 1 : 0, std::max(0, ss[i]->variant))].push_back((int)i);
+      groups[bp_group(ss[i])].push_back((int)i);
     else {
       int rc = launch_bp(ss[i], modes[i], &ntiles[i]);
       if (rc != TG_OK) return rc;
@@ -39,19 +52,13 @@ int batch_bp(tg_batch *b, const std::vector<tg_session *> &ss, const std::vector
     std::vector<int> &idx = kv.second;
     // longest series (most views) first in the tile queue
     std::stable_sort(idx.begin(), idx.end(), [&](int x, int y) { return ss[x]->nviews > ss[y]->nviews; });
-    const int variant = std::get<2>(kv.first);
-    int S, TX, TZ;
-    bp_fast_tile_shape(variant, &S, &TX, &TZ);
     std::vector<BpArgs> jobs;
     long long total = 0;
     int max_views = 1;
     for (int i : idx) {
       BpArgs a = bp_args(ss[i], modes[i]);
-      a.nbx = (a.onx + TX - 1) / TX;
-      const int nbz = (a.onz + TZ - 1) / TZ, nby = (a.ny + S - 1) / S;
-      a.ntiles_xz = a.nbx * nbz;
       a.tile0 = (int)total;
-      total += (long long)a.ntiles_xz * nby;
+      total += bp_group_tiles(kv.first, a);
       ntiles[i] = a.ntiles_xz;
       jobs.push_back(a);
       max_views = std::max(max_views, a.nviews);
@@ -71,7 +78,7 @@ int batch_bp(tg_batch *b, const std::vector<tg_session *> &ss, const std::vector
     bl.ntiles = (int)total;
     bl.counter = b->d_counter;
     bl.max_views = max_views;
-    int rc = launch_bp_batch(bl, std::get<0>(kv.first), std::get<1>(kv.first) != 0, variant, b->st);
+    int rc = launch_bp_group(kv.first, bl, b->st);
     if (rc != TG_OK) return rc;
     TG_CUDA(cudaGetLastError());
     ++*launches;

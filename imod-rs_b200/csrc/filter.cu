@@ -110,10 +110,21 @@ template <bool LOG> __device__ __forceinline__ float4 log4(float4 x, const LogTa
   return r;
 }
 
+__device__ __forceinline__ float finite_abs(float x) { return fabsf(x) <= 3.40282347e+38f ? fabsf(x) : 0.0f; }
+__device__ __forceinline__ float finite_abs4(float4 v) {
+  return fmaxf(fmaxf(finite_abs(v.x), finite_abs(v.y)), fmaxf(finite_abs(v.z), finite_abs(v.w)));
+}
+// raises *range to the block's largest mx (nonnegative floats order as their bits)
+__device__ __forceinline__ void raise_range(float mx, unsigned *range) {
+  const unsigned m = __reduce_max_sync(0xffffffffu, __float_as_uint(mx));
+  if ((threadIdx.x & 31) == 0 && m) atomicMax(range, m);
+}
+
 template <bool LOG>
 __global__ void __launch_bounds__(256) log_sum_kernel(const float *__restrict__ raw, float *__restrict__ logd,
-                                                      long npix, double *partials) {
+                                                      long npix, double *partials, unsigned *range) {
   const int v = blockIdx.y, c = blockIdx.x;
+  float mx = 0.0f;
   __shared__ LogTable lt;
   if (LOG) log_table(lt);
   const size_t base = (size_t)v * npix;
@@ -127,6 +138,7 @@ __global__ void __launch_bounds__(256) log_sum_kernel(const float *__restrict__ 
     float x = raw[base + i];
     if (LOG) logd[base + i] = x = log_sample_fast(x, lt);
     s += (double)x;
+    mx = fmaxf(mx, finite_abs(x));
   }
   const float4 *r4 = reinterpret_cast<const float4 *>(raw + base + a0);
   float4 *l4 = LOG ? reinterpret_cast<float4 *>(logd + base + a0) : nullptr;
@@ -142,17 +154,21 @@ __global__ void __launch_bounds__(256) log_sum_kernel(const float *__restrict__ 
     }
     s += ((double)x.x + (double)x.y) + ((double)x.z + (double)x.w);
     s += ((double)y.x + (double)y.y) + ((double)y.z + (double)y.w);
+    mx = fmaxf(mx, fmaxf(finite_abs4(x), finite_abs4(y)));
   }
   if (i < n4) {
     const float4 x = log4<LOG>(__ldcs(r4 + i), lt);
     if (LOG) l4[i] = x;
     s += ((double)x.x + (double)x.y) + ((double)x.z + (double)x.w);
+    mx = fmaxf(mx, finite_abs4(x));
   }
   for (long k = a1 + threadIdx.x; k < c1; k += blockDim.x) {
     float x = raw[base + k];
     if (LOG) logd[base + k] = x = log_sample_fast(x, lt);
     s += (double)x;
+    mx = fmaxf(mx, finite_abs(x));
   }
+  if (range) raise_range(mx, range);
   __shared__ double red[8];
   for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
   if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
@@ -162,6 +178,29 @@ __global__ void __launch_bounds__(256) log_sum_kernel(const float *__restrict__ 
     for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += red[w];
     partials[(size_t)v * MEAN_CH + c] = t;
   }
+}
+
+// largest finite |in - sub| (a SIRT residual before its filter)
+__global__ void __launch_bounds__(256) residual_range_kernel(const float *__restrict__ in, const float *__restrict__ sub,
+                                                             size_t n, unsigned *range) {
+  const size_t stride = (size_t)gridDim.x * blockDim.x, n4 = n / 4;
+  const float4 *i4 = reinterpret_cast<const float4 *>(in), *s4 = reinterpret_cast<const float4 *>(sub);
+  float mx = 0.0f;
+  auto diff = [](float4 a, float4 b) { return make_float4(a.x - b.x, a.y - b.y, a.z - b.z, a.w - b.w); };
+  size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  for (; i + stride < n4; i += 2 * stride) {  // four 16-byte loads in flight
+    const float4 a = __ldg(i4 + i), b = __ldg(s4 + i), c = __ldg(i4 + i + stride), d = __ldg(s4 + i + stride);
+    mx = fmaxf(mx, fmaxf(finite_abs4(diff(a, b)), finite_abs4(diff(c, d))));
+  }
+  if (i < n4) mx = fmaxf(mx, finite_abs4(diff(__ldg(i4 + i), __ldg(s4 + i))));
+  if (blockIdx.x == 0 && threadIdx.x < n - 4 * n4)
+    mx = fmaxf(mx, finite_abs(__ldg(in + 4 * n4 + threadIdx.x) - __ldg(sub + 4 * n4 + threadIdx.x)));
+  raise_range(mx, range);
+}
+
+void launch_residual_range(const float *in, const float *sub, size_t n, unsigned *range, cudaStream_t st) {
+  const size_t nb = (n / 8 + 255) / 256;
+  residual_range_kernel<<<(unsigned)(nb < 1 ? 1 : nb > 148 * 8 ? 148 * 8 : nb), 256, 0, st>>>(in, sub, n, range);
 }
 
 __global__ void means_final_kernel(const double *partials, long npix, int nviews, float *means) {
@@ -181,9 +220,9 @@ __global__ void view_sums_kernel(const double *partials, int nviews, double *sum
 }
 
 void launch_log_means(const float *raw, float *logd, int npix, int nviews, double *partials,
-                      float *means, cudaStream_t st) {
-  if (logd) log_sum_kernel<true><<<dim3(MEAN_CH, nviews), 256, 0, st>>>(raw, logd, npix, partials);
-  else log_sum_kernel<false><<<dim3(MEAN_CH, nviews), 256, 0, st>>>(raw, nullptr, npix, partials);
+                      float *means, unsigned *range, cudaStream_t st) {
+  if (logd) log_sum_kernel<true><<<dim3(MEAN_CH, nviews), 256, 0, st>>>(raw, logd, npix, partials, range);
+  else log_sum_kernel<false><<<dim3(MEAN_CH, nviews), 256, 0, st>>>(raw, nullptr, npix, partials, range);
   if (means) means_final_kernel<<<(nviews + 127) / 128, 128, 0, st>>>(partials, npix, nviews, means);
 }
 
@@ -258,6 +297,31 @@ template <int STORE> __device__ __forceinline__ void range_track(float &mx, floa
 template <int STORE> __device__ __forceinline__ void range_report(const FilterArgs &a, float mx) {
   if (STORE == TG_STORE_FP16 && mx >= FP16_LIMIT && a.err) atomicOr(a.err, 4);
 }
+
+// OCT staging, rows 2j and 2j+1 of element e: two of the element's eight halves in each
+// plane.  Infinities and NaN are noted in `top` (the largest magnitude bits of any
+// half): the tensor-core back-projector then takes its element-by-element form.
+struct OctWriter {
+  uint32_t *out;     // this row pair's word of element 0 (elements are 4 words apart)
+  size_t plane;      // words to the second plane
+  float scale;
+  uint32_t top = 0;
+  __device__ OctWriter(const FilterArgs &a, int v, int jp)
+      : out(reinterpret_cast<uint32_t *>(a.out) + (((size_t)v * a.rows_alloc + (jp >> 2)) * a.PW) * 4 + (jp & 3)),
+        plane((size_t)a.nviews * a.rows_alloc * a.PW * 4), scale(oct_scale(a.range, a.gain, false)) {}
+  __device__ __forceinline__ void put(int e, float x0, float x1) {  // the samples of both rows
+    x0 = __fmul_rn(x0, scale);
+    x1 = __fmul_rn(x1, scale);
+    const __half2 h = __floats2half2_rn(x0, x1);
+    const uint32_t w = *reinterpret_cast<const uint32_t *>(&h);
+    top = __vmaxu2(top, w & 0x7fff7fffu);
+    out[(size_t)e * 4] = w;
+    out[(size_t)e * 4 + plane] = Pack<TG_STORE_FP16>::h2(__fsub_rn(x0, __low2float(h)), __fsub_rn(x1, __high2float(h)));
+  }
+  __device__ __forceinline__ void report(const FilterArgs &a) const {
+    if ((top & 0xffffu) >= 0x7c00u || (top >> 16) >= 0x7c00u) *a.nonfinite = 1;
+  }
+};
 
 // Value pair (a, b) of element k of a final row, with the reference's fill
 // rule for samples whose left index is out of [0, nx-2] (main.rs:386-406).
@@ -363,6 +427,23 @@ __global__ void __launch_bounds__(256) filter_kernel(FilterArgs a) {
       o0[k] = row0[k];
       if (has1) o0[n + k] = row1[k];
     }
+    return;
+  }
+  if (FMT == FMT_OCT) {  // each element is one sample
+    OctWriter ow(a, v, jp);
+    for (int e = threadIdx.x; e < a.PW; e += blockDim.x) {
+      const int k = e - a.padL;
+      float a0, a1 = 0.0f, b;
+      if (k == n - 1) {
+        a0 = row0[k];
+        if (has1) a1 = row1[k];
+      } else {
+        elem_ab(row0, n, k, a.fill_mode, fillv, a0, b);
+        if (has1) elem_ab(row1, n, k, a.fill_mode, fillv, a1, b);
+      }
+      ow.put(e, a0, a1);
+    }
+    ow.report(a);
     return;
   }
   if (FMT == FMT_ROWPAIR) {
@@ -827,10 +908,7 @@ __device__ __forceinline__ void filter_p2_body(const FilterArgs &a, const int jp
     if (sx0 >= 0 && sx0 < N) return sc(sx0);
     return make_float2(0.0f, 0.0f);
   };
-  // pack into the staging format with the reference's fill rule (main.rs:386-406).
-  // A warp takes 31 consecutive elements e at a time: lane l computes the final
-  // value at k = e - padL straight from the inverse (no second exchange) and
-  // takes the value at k + 1 from lane l + 1; lane 31 only supplies its value.
+  // pack into the staging format with the reference's fill rule (main.rs:386-406)
   const float fillv = a.fill ? a.fill[v] : 0.0f;
   auto fill = [&](int k) -> float2 {
     if (a.fill_mode == TG_FILL_ZERO) return make_float2(0.0f, 0.0f);
@@ -838,6 +916,20 @@ __device__ __forceinline__ void filter_p2_body(const FilterArgs &a, const int jp
     return make_float2(fillv, fillv);
   };
   float hmax = 0.0f;  // largest |value| packed into FP16 by this thread
+  if constexpr (FMT == FMT_OCT) {  // each element is one sample
+    OctWriter ow(a, v, jp);
+    for (int e = t; e < a.PW; e += T) {
+      const int k = e - a.padL;
+      float2 z = k >= 0 && k < N ? fin(k) : fill(k);
+      if (!has1) z.y = 0.0f;
+      ow.put(e, z.x, z.y);
+    }
+    ow.report(a);
+    return;
+  }
+  // the other formats take a sample and the next: a warp takes 31 consecutive elements e at a time: lane l computes the final
+  // value at k = e - padL straight from the inverse (no second exchange) and
+  // takes the value at k + 1 from lane l + 1; lane 31 only supplies its value.
   const size_t row0 = (size_t)v * a.rows_alloc;
   const int lane = t & 31;
   static_assert(T % 32 == 0, "whole warps per row pair");
@@ -986,6 +1078,8 @@ void launch_filter_batch(int n, int fmt, int store, const FilterBatchDev &fb, in
     if (store == TG_STORE_FP32) launch_batch_n<FMT_ROWPAIR, TG_STORE_FP32>(n, fb, nblocks, st);
     else if (store == TG_STORE_FP16) launch_batch_n<FMT_ROWPAIR, TG_STORE_FP16>(n, fb, nblocks, st);
     else launch_batch_n<FMT_ROWPAIR, TG_STORE_BF16>(n, fb, nblocks, st);
+  } else if (fmt == FMT_OCT) {
+    launch_batch_n<FMT_OCT, TG_STORE_FP32>(n, fb, nblocks, st);
   } else {
     if (store == TG_STORE_FP32) launch_batch_n<FMT_SINGLE, TG_STORE_FP32>(n, fb, nblocks, st);
     else if (store == TG_STORE_FP16) launch_batch_n<FMT_SINGLE, TG_STORE_FP16>(n, fb, nblocks, st);
@@ -998,6 +1092,8 @@ void launch_filter(const FilterArgs &a, cudaStream_t st) {
     if (a.store == TG_STORE_FP32) launch_f<FMT_ROWPAIR, TG_STORE_FP32>(a, st);
     else if (a.store == TG_STORE_FP16) launch_f<FMT_ROWPAIR, TG_STORE_FP16>(a, st);
     else launch_f<FMT_ROWPAIR, TG_STORE_BF16>(a, st);
+  } else if (a.fmt == FMT_OCT) {
+    launch_f<FMT_OCT, TG_STORE_FP32>(a, st);
   } else {
     if (a.store == TG_STORE_FP32) launch_f<FMT_SINGLE, TG_STORE_FP32>(a, st);
     else if (a.store == TG_STORE_FP16) launch_f<FMT_SINGLE, TG_STORE_FP16>(a, st);

@@ -8,8 +8,8 @@
 //     same form share one launch per phase over a block table);
 //   * residual filter: series with the same register-resident FFT width,
 //     staging format and precision share one launch;
-//   * back-projection: one persistent launch per (precision, z-factor, tile
-//     variant) group with a longest-first tile queue, as in batch_bp;
+//   * back-projection: one launch per group (bp_group) with a longest-first tile
+//     queue, as in batch_bp;
 // series that fit no group (local alignment, general kernels, other widths)
 // get their own launches inside the same plan.  Each group kernel runs the
 // per-series body on each block's own series, so every series' result is the
@@ -50,6 +50,7 @@ void round_plan_release(RoundPlan &p, cudaStream_t st) {
   p.fi.clear();
   p.bp.clear();
   p.fp_single.clear();
+  p.scaled.clear();
   p.fi_single.clear();
   p.bp_single.clear();
   p.host.clear();
@@ -69,6 +70,7 @@ int round_plan_build(RoundPlan &p, const std::vector<tg_session *> &ss, const st
   p.fi.clear();
   p.bp.clear();
   p.fp_single.clear();
+  p.scaled.clear();
   p.fi_single.clear();
   p.bp_single.clear();
   p.launches = 0;
@@ -112,6 +114,7 @@ int round_plan_build(RoundPlan &p, const std::vector<tg_session *> &ss, const st
   // residual filter groups
   std::map<std::tuple<int, int, int>, std::vector<FilterArgs>> fig;
   for (tg_session *s : ss) {
+    if (s->mma_steps) p.scaled.push_back(s);
     FilterArgs f = filter_args(s, true);
     const int n = filter_batch_width(f);
     if (n == 0) p.fi_single.push_back(s);
@@ -131,30 +134,23 @@ int round_plan_build(RoundPlan &p, const std::vector<tg_session *> &ss, const st
     p.fi.push_back(g);
   }
   // back-projection groups (batch_bp's grouping, SIRT update mode)
-  std::map<std::tuple<int, int, int>, std::vector<tg_session *>> bpg;
+  std::map<BpGroup, std::vector<tg_session *>> bpg;
   for (tg_session *s : ss) {
-    if (s->fast) bpg[std::make_tuple(s->store, s->zf_any ? 1 : 0, std::max(0, s->variant))].push_back(s);
+    if (s->fast) bpg[bp_group(s)].push_back(s);
     else p.bp_single.push_back(s);
   }
   for (auto &kv : bpg) {
     std::vector<tg_session *> &mem = kv.second;
     std::stable_sort(mem.begin(), mem.end(), [](tg_session *x, tg_session *y) { return x->nviews > y->nviews; });
     RoundPlan::Bp g{};
-    g.store = std::get<0>(kv.first);
-    g.zf = std::get<1>(kv.first);
-    g.variant = std::get<2>(kv.first);
-    int S, TX, TZ;
-    bp_fast_tile_shape(g.variant, &S, &TX, &TZ);
+    g.group = kv.first;
     std::vector<BpArgs> jobs;
     long long total = 0;
     g.max_views = 1;
     for (tg_session *s : mem) {
       BpArgs a = bp_args(s, 2);
-      a.nbx = (a.onx + TX - 1) / TX;
-      const int nbz = (a.onz + TZ - 1) / TZ, nby = (a.ny + S - 1) / S;
-      a.ntiles_xz = a.nbx * nbz;
       a.tile0 = (int)total;
-      total += (long long)a.ntiles_xz * nby;
+      total += bp_group_tiles(kv.first, a);
       jobs.push_back(a);
       g.max_views = std::max(g.max_views, a.nviews);
     }
@@ -189,6 +185,13 @@ int round_plan_issue(RoundPlan &p, cudaStream_t st) {
                                        reinterpret_cast<const int *>(d + g.copy), g.ncopy,
                                        reinterpret_cast<const int *>(d + g.fpb), g.nfp, st);
   for (tg_session *s : p.fp_single) launches += launch_reproject(fp_args(s), st);
+  for (tg_session *s : p.scaled) {
+    const cudaStream_t own = s->st;
+    s->st = st;
+    const int rc = stage_residual_range(s, &launches);
+    s->st = own;
+    if (rc != TG_OK) return rc;
+  }
   for (const RoundPlan::Fi &g : p.fi) {
     FilterBatchDev fb{reinterpret_cast<const FilterArgs *>(d + g.jobs), reinterpret_cast<const int *>(d + g.blk),
                       g.njobs};
@@ -206,7 +209,7 @@ int round_plan_issue(RoundPlan &p, cudaStream_t st) {
     bl.ntiles = g.ntiles;
     bl.counter = reinterpret_cast<int *>(d + g.counter);
     bl.max_views = g.max_views;
-    const int rc = launch_bp_batch(bl, g.store, g.zf != 0, g.variant, st);
+    const int rc = launch_bp_group(g.group, bl, st);
     if (rc != TG_OK) return rc;
     ++launches;
   }

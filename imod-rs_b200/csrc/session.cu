@@ -155,7 +155,7 @@ static void free_session(tg_session *s) {
   void *ptrs[] = {s->d_raw, s->d_logd, s->d_means, s->d_vol, s->d_sino, s->d_tmp, s->d_volg, s->d_volh, s->d_maxbits, s->d_mpart, s->d_pairs,
                   s->d_part, s->d_slice_stats, s->d_stats3, s->d_vg, s->d_vg2, s->d_weights,
                   s->d_conv, s->d_stretch, s->d_tw, s->d_err, s->d_lvinfo, s->d_lgoff, s->d_lxs,
-                  s->d_lys, s->d_lgdx, s->d_lgdy, s->d_ltab, s->d_xtb, s->d_lbnd, s->d_half};
+                  s->d_lys, s->d_lgdx, s->d_lgdy, s->d_ltab, s->d_xtb, s->d_lbnd, s->d_half, s->d_tmap};
   for (void *p : ptrs)
     if (p) cudaFree(p);
   for (auto &e : s->ev)
@@ -169,7 +169,7 @@ void free_session_async(tg_session *s, cudaStream_t after) {
   void *ptrs[] = {s->d_raw, s->d_logd, s->d_means, s->d_vol, s->d_sino, s->d_tmp, s->d_volg, s->d_volh, s->d_maxbits, s->d_mpart, s->d_pairs,
                   s->d_part, s->d_slice_stats, s->d_stats3, s->d_vg, s->d_vg2, s->d_weights,
                   s->d_conv, s->d_stretch, s->d_tw, s->d_err, s->d_lvinfo, s->d_lgoff, s->d_lxs,
-                  s->d_lys, s->d_lgdx, s->d_lgdy, s->d_ltab, s->d_xtb, s->d_lbnd, s->d_half};
+                  s->d_lys, s->d_lgdx, s->d_lgdy, s->d_ltab, s->d_xtb, s->d_lbnd, s->d_half, s->d_tmap};
   for (void *p : ptrs)
     if (p) cudaFreeAsync(p, after);
   for (auto &e : s->ev)
@@ -285,6 +285,10 @@ BpArgs bp_args(tg_session *s, int mode) {
   a.loc = local_dev(s);
   a.wait_limit_ns = s->wait_limit_ns;
   a.fault_skip_stage = s->fault_skip_stage;
+  a.nonfinite = s->d_err + 1;
+  a.range = reinterpret_cast<unsigned *>(s->d_err + 2);
+  a.gain = s->oct_gain;
+  a.tmap = s->d_tmap;
   return a;
 }
 
@@ -312,16 +316,23 @@ FilterArgs filter_args(tg_session *s, bool residual) {
   f.inv_n = 1.0f / (float)s->nx;
   f.plan = s->plan;
   f.err = s->d_err;
+  f.nonfinite = s->d_err + 1;
+  f.range = reinterpret_cast<unsigned *>(s->d_err + 2);
+  f.gain = s->oct_gain;
   return f;
 }
 
 int launch_bp(tg_session *s, int mode, int *ntiles) {
   BpArgs a = bp_args(s, mode);
-  if (s->fast) return launch_bp_fast(a, s->store, fast_zf(s), s->variant < 0 ? 0 : s->variant, s->st, ntiles);
+  auto rows = [&](const BpArgs &b, int *nt) {
+    if (s->mma_steps) return launch_bp_mma(b, s->mma_steps, s->st, nt);
+    return launch_bp_fast(b, s->store, fast_zf(s), s->variant < 0 ? 0 : s->variant, s->st, nt);
+  };
+  if (s->fast) return rows(a, ntiles);
   if (s->xt_split) {  // per-row view sums, then the two-row blend of every voxel
     BpArgs r = bp_args(s, 1);
     r.vol = s->xtb;
-    int rc = launch_bp_fast(r, s->store, fast_zf(s), s->variant < 0 ? 0 : s->variant, s->st, nullptr);
+    int rc = rows(r, nullptr);
     if (rc != TG_OK) return rc;
     return launch_xt_blend(a, s->xtb, s->sin_xt_common, s->st, ntiles);
   }
@@ -332,7 +343,7 @@ int launch_bp(tg_session *s, int mode, int *ntiles) {
 // Times each fast tile variant once on (the first 64 slices of) this series and
 // keeps the fastest (process-wide cache keyed by the series shape).
 int autotune(tg_session *s) {
-  if (!s->fast && !s->xt_split) { s->variant = 0; return TG_OK; }
+  if ((!s->fast && !s->xt_split) || s->mma_steps) { s->variant = 0; return TG_OK; }
   if (const char *env = getenv("TG_BP_VARIANT")) {  // fixed tile shape (profiling, tuning)
     int v = atoi(env);
     if (v >= 0 && v < bp_fast_variants()) { s->variant = v; return TG_OK; }
@@ -378,7 +389,7 @@ int autotune(tg_session *s) {
 }
 
 int tune_lookup(tg_session *s) {
-  if (!s->fast && !s->xt_split) return 0;
+  if ((!s->fast && !s->xt_split) || s->mma_steps) return 0;
   if (const char *env = getenv("TG_BP_VARIANT")) {
     int v = atoi(env);
     if (v >= 0 && v < bp_fast_variants()) return v;
@@ -416,11 +427,29 @@ FpArgs fp_args(tg_session *s) {
   return f;
 }
 
+// log10 and per-view means (main.rs:608-623).  On the tensor-core path the error words
+// behind the first start over: d_err[1] is FilterArgs::nonfinite, d_err[2] its range.
+static int stage_log_means(tg_session *s) {
+  if (s->mma_steps) TG_CUDA(cudaMemsetAsync(s->d_err + 1, 0, 8, s->st));
+  launch_log_means(s->d_raw, s->d_logd, s->nx * s->ny, s->nz, s->d_mpart, s->means_pinned ? nullptr : s->d_means,
+                   s->mma_steps ? reinterpret_cast<unsigned *>(s->d_err + 2) : nullptr, s->st);
+  return TG_OK;
+}
+
+int stage_residual_range(tg_session *s, int *launches) {
+  if (!s->mma_steps) return TG_OK;
+  unsigned *range = reinterpret_cast<unsigned *>(s->d_err + 2);
+  TG_CUDA(cudaMemsetAsync(range, 0, sizeof(unsigned), s->st));
+  launch_residual_range(s->d_logd ? s->d_logd : s->d_raw, s->d_sino, (size_t)s->nx * s->ny * s->nviews, range, s->st);
+  *launches += 1;
+  return TG_OK;
+}
+
 int stage_front(tg_session *s, int *launches) {
+  int rc;
   // every run starts from the uploaded projections: log10 into d_logd (--log) and the
   // per-view means, as main.rs:608-623 does before each reconstruction
-  launch_log_means(s->d_raw, s->d_logd, s->nx * s->ny, s->nz, s->d_mpart, s->means_pinned ? nullptr : s->d_means,
-                   s->st);
+  if ((rc = stage_log_means(s)) != TG_OK) return rc;
   *launches += 2;
   launch_filter(filter_args(s, false), s->st);
   *launches += 1;
@@ -596,7 +625,13 @@ int tg::session_create_ex(const tg_geometry *g, const tg_options *opt, cudaMemPo
     }
     s->xt_fast = ok && bp_xtilt_supported(s->onx, msx, mext);
   }
-  s->fmt = s->fast || s->xt_split ? FMT_ROWPAIR : FMT_SINGLE;
+  // FP32 staging of R-weighted rows back-projects on the tensor cores; without R-weighting the
+  // result is the reference's bit for bit, which the fast kernel keeps.
+  bool oct = (s->fast || s->xt_split) && s->store == TG_STORE_FP32 && !opt->no_weight;
+  if (const char *env = getenv("TG_BP_VARIANT")) oct = oct && atoi(env) == bp_fast_variants();  // fixed kernel
+  else oct = oct && bp_mma_pays(s->onx, s->onz, s->ny, s->nviews);
+  s->fmt = !s->fast && !s->xt_split ? FMT_SINGLE : oct ? FMT_OCT : FMT_ROWPAIR;
+  if (oct) s->mma_steps = bp_mma_steps(vg);
 
   // cosine stretch factors (main.rs:446-460); the reference indexes
   // tilt_angles[p] for every section p < nz and panics if the file is short.
@@ -633,10 +668,13 @@ int tg::session_create_ex(const tg_geometry *g, const tg_options *opt, cudaMemPo
     int needL = std::max(0, -kmin), needR = std::max(0, kmax - (s->nx - 1));
     s->padL = ((needL + 3) + 1) & ~1;
     int padR = needR + 6;
+    if (s->fmt == FMT_OCT) padR = std::max(padR, 32 - s->padL - s->nx);  // a whole staged window at least
     s->PW = (s->padL + s->nx + padR + 1) & ~1;
   }
   const int ra = bp_fast_row_align();  // a tile's row pairs never pass the allocation
-  s->rows_alloc = s->fmt == FMT_ROWPAIR ? ((s->ny + ra - 1) / ra) * (ra / 2) : s->ny;
+  s->rows_alloc = s->fmt == FMT_ROWPAIR ? ((s->ny + ra - 1) / ra) * (ra / 2)
+                  : s->fmt == FMT_OCT   ? (s->ny + 15) / 16 * 2
+                                        : s->ny;
 
   // FFT plan or circulant fallback
   s->use_conv = !fft_plan(s->nx, &s->plan);
@@ -662,6 +700,7 @@ int tg::session_create_ex(const tg_geometry *g, const tg_options *opt, cudaMemPo
     a.onz = s->onz;
     for (int v = 0; v < bp_fast_variants(); ++v) ntiles = std::max(ntiles, bp_fast_ntiles(a, v));
     ntiles = std::max(ntiles, ((s->onx + 31) / 32) * ((s->onz + 15) / 16));
+    if (s->fmt == FMT_OCT) ntiles = std::max(ntiles, bp_mma_ntiles(s->onx, s->onz));
   }
   s->ntiles_cap = ntiles;
   if ((rc = dalloc(s, &s->d_raw, nproj * 4)) || (rc = dalloc(s, &s->d_means, (size_t)s->nz * 4)) ||
@@ -673,6 +712,7 @@ int tg::session_create_ex(const tg_geometry *g, const tg_options *opt, cudaMemPo
       (rc = dalloc(s, &s->d_weights, (size_t)s->nx * 4)) || (rc = dalloc(s, &s->d_tw, (size_t)s->nx * 16)) ||
       (rc = dalloc(s, &s->d_stretch, (size_t)s->nviews * 4)) || (rc = dalloc(s, &s->d_err, 16)))
     return fail(rc);
+  if (s->mma_steps && (rc = dalloc(s, &s->d_tmap, 128))) return fail(rc);
   if (opt->log_transform && (rc = dalloc(s, &s->d_logd, nproj * 4))) return fail(rc);
   if (!opt->gpu_compat && opt->sirt_iters > 0 && (rc = dalloc(s, &s->d_sino, nproj * 4))) return fail(rc);
   if (!opt->gpu_compat && opt->fake_sirt > 0 && (rc = dalloc(s, &s->d_tmp, nvol * 4))) return fail(rc);
@@ -742,6 +782,11 @@ int tg::session_create_ex(const tg_geometry *g, const tg_options *opt, cudaMemPo
     if ((ce = cudaMemcpyAsync(s->d_conv, h.data(), h.size() * 4, cudaMemcpyHostToDevice, s->st)))
       return fail(cuda_fail(ce, "copy"));
   }
+  {
+    double w2 = 0.0;
+    for (float w : wt) w2 += (double)w * w;
+    s->oct_gain = (float)std::max(1.0, sqrt(w2)) * (opt->cosine_cubic ? 1.25f : 1.0f);
+  }
   // on the session's stream (after its stream-ordered allocations); pageable
   // sources have been staged when each call returns; synchronised below
   if ((ce = cudaMemcpyAsync(s->d_weights, wt.data(), wt.size() * 4, cudaMemcpyHostToDevice, s->st)) ||
@@ -750,6 +795,13 @@ int tg::session_create_ex(const tg_geometry *g, const tg_options *opt, cudaMemPo
       (ce = cudaMemcpyAsync(s->d_vg2, vg2.data(), vg2.size() * 16, cudaMemcpyHostToDevice, s->st)) ||
       (ce = cudaMemcpyAsync(s->d_stretch, stretch.data(), stretch.size() * 4, cudaMemcpyHostToDevice, s->st)))
     return fail(cuda_fail(ce, "cudaMemcpy(setup)"));
+  unsigned char tmap[128];
+  if (s->mma_steps) {
+    BpArgs a = bp_args(s, 0);
+    bp_mma_plan(a);
+    if ((rc = bp_mma_tensor_map(s->d_pairs, s->nviews, s->rows_alloc, s->PW, a.nper, s->mma_steps, tmap)) != TG_OK) return fail(rc);
+    if ((ce = cudaMemcpyAsync(s->d_tmap, tmap, 128, cudaMemcpyHostToDevice, s->st))) return fail(cuda_fail(ce, "cudaMemcpy(setup)"));
+  }
   if (!any_stretch) {
     if (pool) cudaFreeAsync(s->d_stretch, s->st);
     else cudaFree(s->d_stretch);
@@ -793,6 +845,8 @@ namespace tg {
 int sirt_iterations(tg_session *s, int n) {
   auto one_iter = [&]() -> int {
     s->iter_launches = launch_reproject(fp_args(s), s->st) + 1 + bp_launch_count(s);
+    const int rc = stage_residual_range(s, &s->iter_launches);
+    if (rc != TG_OK) return rc;
     launch_filter(filter_args(s, true), s->st);
     return launch_bp(s, 2, nullptr);
   };
@@ -928,8 +982,7 @@ int tg_sirt_restore(tg_session *s, const float *host_volume, int32_t iterations_
   if (s->variant < 0 && (rc = autotune(s)) != TG_OK) return rc;
   s->timed = false;
   // the log and the per-view means the iterations read (main.rs:608-623)
-  launch_log_means(s->d_raw, s->d_logd, s->nx * s->ny, s->nz, s->d_mpart, s->means_pinned ? nullptr : s->d_means,
-                   s->st);
+  if ((rc = stage_log_means(s)) != TG_OK) return rc;
   TG_CUDA(cudaMemcpyAsync(s->d_vol, host_volume, (size_t)s->onx * s->onz * s->ny * 4, cudaMemcpyHostToDevice,
                           s->st));
   TG_CUDA(cudaStreamSynchronize(s->st));  // the pageable source may be reused on return
@@ -1080,7 +1133,7 @@ int tg_session_kernel_info(tg_session *s, int32_t *fast, int32_t *variant, int32
   if (!s) return TG_ERR_INVALID_ARG;
   // 2: staged x-tilt kernel, 3: fast kernel's row sums + blend, 0: general kernel
   if (fast) *fast = s->fast ? 1 : s->xt_split ? 3 : s->xt_fast ? 2 : 0;
-  if (variant) *variant = s->variant;
+  if (variant) *variant = s->mma_steps ? bp_fast_variants() : s->variant;
   if (fmt) *fmt = s->fmt;
   if (padL) *padL = s->padL;
   if (PW) *PW = s->PW;
@@ -1093,7 +1146,7 @@ int tg_session_view_sums(tg_session *s, double *sums) {
   TG_CUDA(cudaSetDevice(s->dev));
   double *d = nullptr;
   TG_CUDA(cudaMallocAsync((void **)&d, (size_t)s->nz * sizeof(double), s->st));
-  launch_log_means(s->d_raw, s->d_logd, s->nx * s->ny, s->nz, s->d_mpart, nullptr, s->st);
+  launch_log_means(s->d_raw, s->d_logd, s->nx * s->ny, s->nz, s->d_mpart, nullptr, nullptr, s->st);
   launch_view_sums(s->d_mpart, s->nz, d, s->st);
   cudaError_t e = cudaGetLastError();
   if (e == cudaSuccess) e = cudaMemcpyAsync(sums, d, (size_t)s->nz * sizeof(double), cudaMemcpyDeviceToHost, s->st);
@@ -1133,13 +1186,13 @@ int tg_session_inject_wait_fault(tg_session *s, int32_t skip_stage, uint32_t wai
 }
 
 int tg_session_set_variant(tg_session *s, int32_t variant) {
-  if (!s || variant < -1 || variant >= bp_fast_variants()) return TG_ERR_INVALID_ARG;
-  s->variant = variant;
+  if (!s || variant < -1 || variant >= bp_fast_variants() + (s->mma_steps ? 1 : 0)) return TG_ERR_INVALID_ARG;
+  if (!s->mma_steps) s->variant = variant;  // the tensor-core kernel has one tile shape
   return TG_OK;
 }
 
 const char *tg_variant_name(int32_t v) {
-  return (v >= 0 && v < bp_fast_variants()) ? bp_fast_variant_name(v) : "general";
+  return v == bp_fast_variants() ? "tcgen05-hex126" : (v >= 0 && v < bp_fast_variants()) ? bp_fast_variant_name(v) : "general";
 }
 
 // ---- the reference's GPU seam (apps/tilt/src/gpu.rs) ----

@@ -19,6 +19,9 @@ struct tg_session {  // one tilt series resident on a device
   // x-tilt shared by all views: the fast kernel sums every projection row over the
   // views into xtb, then launch_xt_blend blends two rows per voxel into the volume
   bool xt_split = false;
+  int mma_steps = 0;       // fast or row-sum path on the tensor-core back-projector: its K steps (else 0)
+  void *d_tmap = nullptr;  // TMA map of d_pairs on that path
+  float oct_gain = 1.0f;   // oct_scale's gain on that path
   float *xtb = nullptr;    // row sums (d_xtb, or the reprojector's FP32 copy, which is dead then)
   float *d_xtb = nullptr;
   int fp_fast = 0;  // reprojector: 0 general, 1 fast (no x-tilt), 2 fast with x-tilt
@@ -91,9 +94,21 @@ int launch_bp(tg_session *s, int mode, int *ntiles);
 inline int bp_launch_count(const tg_session *s) { return s->xt_split ? 2 : 1; }
 // position form of the fast kernel: 2 with x-tilt (row sums), else whether z-factors apply
 inline int fast_zf(const tg_session *s) { return s->xt_split ? 2 : s->zf_any ? 1 : 0; }
+// Series whose back-projections share a batched launch: the fast kernel's by z-factor and
+// tile variant (each keeps the shape tuned for it), the tensor-core kernel's by K steps
+using BpGroup = std::tuple<int, int, int>;  // (storage, z-factor or K steps, variant or -1: tensor cores)
+inline BpGroup bp_group(const tg_session *s) {
+  if (s->mma_steps) return BpGroup(s->store, s->mma_steps, -1);
+  return BpGroup(s->store, s->zf_any ? 1 : 0, s->variant < 0 ? 0 : s->variant);
+}
+// fills a's tile grid for its group's kernel; returns its tiles
+long long bp_group_tiles(const BpGroup &g, BpArgs &a);
+int launch_bp_group(const BpGroup &g, const BatchLaunch &bl, cudaStream_t st);
 int autotune(tg_session *s);
 // the tile variant already tuned for this shape (or pinned by TG_BP_VARIANT), else -1
 int tune_lookup(tg_session *s);
+// before the filter of a SIRT residual on the tensor-core path: the residual's range
+int stage_residual_range(tg_session *s, int *launches);
 // log10 + per-view means, then the filter stage of the WBP pass
 int stage_front(tg_session *s, int *launches);
 // fake-SIRT passes, output transform (when the volume was stored raw) and statistics;
@@ -103,8 +118,7 @@ inline int sirt_iters(const tg_session *s) { return s->o.gpu_compat ? 0 : s->o.s
 inline int fake_passes(const tg_session *s) { return s->o.gpu_compat ? 0 : s->o.fake_sirt; }
 inline int first_mode(const tg_session *s) { return (sirt_iters(s) > 0 || fake_passes(s) > 0) ? 1 : 0; }
 
-// One persistent back-projection launch per (storage, z-factor) group of
-// fast-path series, on b->st; other series get their own launch.  ntiles[i]
+// One back-projection launch per group (bp_group) of fast-path series, on b->st; other series get their own launch.  ntiles[i]
 // receives the partial-stat tile count written for ss[i] (used when
 // modes[i] == 0).  Job and tile tables are copied stream-ordered, so calls may
 // follow each other on the same stream without waiting.
@@ -124,11 +138,11 @@ struct RoundPlan {
   size_t cap = 0;
   struct Fp { int key, njobs, nabs, ncopy, nfp; size_t jobs, abs, copy, fpb; };
   struct Fi { int n, fmt, store, njobs, nblk; size_t jobs, blk; };
-  struct Bp { int store, zf, variant, njobs, ntiles, max_views; size_t jobs, counter; };
+  struct Bp { BpGroup group; int njobs, ntiles, max_views; size_t jobs, counter; };
   std::vector<Fp> fp;
   std::vector<Fi> fi;
   std::vector<Bp> bp;
-  std::vector<tg_session *> fp_single, fi_single, bp_single;
+  std::vector<tg_session *> fp_single, fi_single, bp_single, scaled;
   cudaGraphExec_t exec = nullptr;
   int launches = 0;  // kernels of one issue
 };

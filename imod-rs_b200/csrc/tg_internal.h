@@ -23,9 +23,13 @@ namespace tg {
 // ([view][row-pair][PW]): FP32 float4 (a0, a1, b0, b1), FP16/BF16 uint2
 // (h2(a0,a1), h2(d0,d1)).  SINGLE keeps one row per element ([view][row][PW]):
 // FP32 float2 (a, b), FP16/BF16 uint32 h2(a, d).
-enum Fmt { FMT_ROWPAIR = 0, FMT_SINGLE = 1, FMT_ROWS = 2 /* plain filtered rows, in place */ };
+// OCT is FP32 staging for the tensor-core back-projector: 8 consecutive rows per
+// element, [plane][view][block of 8 rows][PW][8] halves; planes 0 and 1 hold the FP16
+// leading part and remainder of row[k] * oct_scale, k outside [0, nx) the fill's.
+enum Fmt { FMT_ROWPAIR = 0, FMT_SINGLE = 1, FMT_ROWS = 2 /* plain filtered rows, in place */, FMT_OCT = 3 };
 
 inline int elem_bytes(int fmt, int store) {
+  if (fmt == FMT_OCT) return 32;  // both planes
   if (fmt == FMT_ROWPAIR) return store == TG_STORE_FP32 ? 16 : 8;
   return store == TG_STORE_FP32 ? 8 : 4;
 }
@@ -37,9 +41,29 @@ struct StatPartial {
 
 // ---- log transform + per-view means (main.rs:608-623) ----
 // logd == nullptr: means of raw; else logd = log10(max(raw, 0.001)) and its means
-// (means == nullptr: partial sums only)
+// (means == nullptr: partial sums only).  range (if given): raised to the largest finite
+// magnitude, as float bits
 void launch_log_means(const float *raw, float *logd, int npix, int nviews, double *partials,
-                      float *means, cudaStream_t st);
+                      float *means, unsigned *range, cudaStream_t st);
+// the same of the residual in - sub of n values
+void launch_residual_range(const float *in, const float *sub, size_t n, unsigned *range, cudaStream_t st);
+// Power of two that the filtered rows of an OCT series are staged times: range is the
+// largest finite magnitude of the filter's input, gain a bound of the filter's amplification
+// (the 2-norm of the weights bounds the impulse response's 1-norm), so scaled rows stay
+// below 2^15; FP16 then holds 22 bits of every value down to 2^-17 of that bound.
+__host__ __device__ inline float oct_scale(const unsigned *range, float gain, bool inverse) {
+#ifdef __CUDA_ARCH__
+  const float m = fminf(__uint_as_float(*range) * gain, 1.0e38f);
+  if (!(m > 0.0f)) return 1.0f;
+  int e;
+  frexpf(m, &e);  // m < 2^e
+  e = max(e, -100);
+  return ldexpf(1.0f, inverse ? e - 15 : 15 - e);
+#else
+  (void)range, (void)gain, (void)inverse;
+  return 1.0f;
+#endif
+}
 // per-view f64 sums from the partials of launch_log_means
 void launch_view_sums(const double *partials, int nviews, double *sums, cudaStream_t st);
 
@@ -69,6 +93,9 @@ struct FilterArgs {
   float inv_n;
   FftPlanDev plan;
   int *err;                 // session error word: bit 2 set when a value exceeds the FP16 range
+  int *nonfinite;           // OCT: set to 1 when a staged value is infinite or NaN
+  const unsigned *range;    // OCT: see oct_scale
+  float gain;
 };
 void launch_filter(const FilterArgs &a, cudaStream_t st);
 // Twiddles of the register-resident filter kernel for rows of n samples, per
@@ -119,6 +146,13 @@ struct BpArgs {
   // test hook (tg_session_inject_wait_fault): the producer issues no copy for this
   // stage of each tile, so the consumers' wait on it runs out; -1: none
   int fault_skip_stage;
+  // tensor-core kernel: slices per tile (set by bp_mma_plan), and this pass's
+  // FilterArgs::nonfinite, range and gain
+  int nper;
+  const int *nonfinite;
+  const unsigned *range;
+  const void *tmap;         // TMA map of pairs (bp_mma_tensor_map), in device memory
+  float gain;
   int pad_;
 };
 // A persistent back-projection launch over the tiles of several series.  Tile t
@@ -141,6 +175,15 @@ int launch_bp_fast(const BpArgs &a, int store, int zf, int variant, cudaStream_t
                    int *ntiles_out);
 int bp_fast_variants();
 const char *bp_fast_variant_name(int v);
+// Tensor-core kernel (backproject_mma.cu): the fast kernel's cases with FP32 staging and
+// R-weighting; OCT format.  vg: the views' (cos, sin, zf, cos_xt).
+int bp_mma_steps(const std::vector<float4> &vg);
+long long bp_mma_plan(BpArgs &a);  // fills the tile grid (nbx, ntiles_xz, nper); returns the tiles
+int bp_mma_ntiles(int onx, int onz);
+bool bp_mma_pays(int onx, int onz, int ny, int nviews);
+int bp_mma_tensor_map(void *pairs, int nviews, int rows_alloc, int PW, int nper, int steps, unsigned char out[128]);
+int launch_bp_mma(const BpArgs &a, int steps, cudaStream_t st, int *ntiles_out);
+int launch_bp_mma_batch(const BatchLaunch &bl, int steps, cudaStream_t st);
 // General kernel: x-tilt, z-factor, local alignment, SINGLE format.
 int launch_bp_general(const BpArgs &a, int store, cudaStream_t st, int *ntiles_out);
 // x-tilt back-projection with staged rows (no local alignment); same tile grid
