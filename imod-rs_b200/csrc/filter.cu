@@ -14,6 +14,7 @@
 #include <mutex>
 
 #include <algorithm>
+#include <complex>
 #include <cstdlib>
 #include <cstring>
 
@@ -339,6 +340,70 @@ __device__ __forceinline__ void elem_ab(const float *row, int nx, int k, int fil
   }
 }
 
+// B[k] = sum over m = 0, 1, ... of h[(k - m) mod n] * A[m] (both rows of a pair), one fused
+// multiply-add per term in that order.  A thread owns CONV_R consecutive outputs: their
+// taps are a window of CONV_R values that slides by one per m, so a term costs one packed fma
+// for both rows, one tap load per CONV_R of them, and a share of a broadcast of A (one
+// output per thread took six instructions and two loads per term).  717 rows x 77 views of 1023
+// samples: 13.4 -> 3.7 ms, the fused multiply-adds alone 1.6; 512 x 61 of 2001: 29.4 -> 7.9.  H: the taps of every distance
+// in rows of equal (j mod 8), so that neighbouring threads read neighbouring words.
+constexpr int CONV_R = 8;
+__host__ __device__ inline int conv_off(int n) { return ((n - 1 + CONV_R - 1) / CONV_R + 1) * CONV_R; }
+__host__ __device__ inline int conv_cols(int n) { return (n + conv_off(n)) / CONV_R + 1; }
+inline bool conv_tiled(int n) { return 16 * (size_t)n + 4 * CONV_R * (size_t)conv_cols(n) <= 220 * 1024; }
+__device__ __forceinline__ void circulant(const float2 *A, float2 *B, float *H, const float *__restrict__ h, int n) {
+  const int cols = conv_cols(n), off = conv_off(n);  // tap j at index j + off
+  for (int i = threadIdx.x; i < CONV_R * cols; i += blockDim.x) {
+    const int j = (i - off) % n;
+    H[(i & 7) * cols + (i >> 3)] = __ldg(&h[j < 0 ? j + n : j]);
+  }
+  __syncthreads();
+  for (int k0 = CONV_R * threadIdx.x; k0 < n; k0 += CONV_R * blockDim.x) {
+    uint64_t s[CONV_R];
+    float w[CONV_R];
+    const float *col = H + ((k0 + off) >> 3);  // tap k0 - m: row (-m) mod 8, column (k0 + off - m) / 8
+#pragma unroll
+    for (int r = 0; r < CONV_R; ++r) {
+      s[r] = 0;
+      w[r] = col[r * cols];
+    }
+    for (int m0 = 0; m0 < n; m0 += CONV_R) {
+#pragma unroll
+      for (int u = 0; u < CONV_R; ++u) {  // m = m0 + u: output r takes the tap in w[(r - u) mod 8]
+        if (m0 + u < n) {
+          const float2 z = A[m0 + u];
+          const uint64_t z2 = pk2(z.x, z.y);
+#pragma unroll
+          for (int r = 0; r < CONV_R; ++r) {
+            const float t = w[(r - u) & (CONV_R - 1)];
+            s[r] = fma2(pk2(t, t), z2, s[r]);
+          }
+        }
+        w[CONV_R - 1 - u] = col[(CONV_R - 1 - u) * cols - 1];  // tap k0 - m0 - u - 1
+      }
+      --col;
+    }
+#pragma unroll
+    for (int r = 0; r < CONV_R; ++r)
+      if (k0 + r < n) B[k0 + r] = up2(s[r]);
+  }
+}
+// the same for rows too long for H in shared memory: one output per thread
+__device__ __forceinline__ void circulant_long(const float2 *A, float2 *B, const float *__restrict__ h, int n) {
+  for (int k = threadIdx.x; k < n; k += blockDim.x) {
+    float s0 = 0.f, s1 = 0.f;
+    for (int m = 0; m < n; ++m) {
+      int d = k - m;
+      d += d < 0 ? n : 0;
+      const float t = __ldg(&h[d]);
+      const float2 z = A[m];
+      s0 = fmaf(t, z.x, s0);
+      s1 = fmaf(t, z.y, s1);
+    }
+    B[k] = make_float2(s0, s1);
+  }
+}
+
 // One CTA per (row pair, view).  Rows 2j and 2j+1 are packed as the real and
 // imaginary part of one complex FFT: with a real, even weight the inverse
 // returns both filtered rows at once.
@@ -381,18 +446,8 @@ __global__ void __launch_bounds__(256) filter_kernel(FilterArgs a) {
     } else {
       // n without a radix-2/3/5/7 plan: circulant convolution with the
       // inverse transform of the weights (h already includes 1/n).
-      for (int k = threadIdx.x; k < n; k += blockDim.x) {
-        float s0 = 0.f, s1 = 0.f;
-        for (int m = 0; m < n; ++m) {
-          int d = k - m;
-          d += d < 0 ? n : 0;
-          float h = __ldg(&a.conv_h[d]);
-          float2 z = A[m];
-          s0 = fmaf(h, z.x, s0);
-          s1 = fmaf(h, z.y, s1);
-        }
-        B[k] = make_float2(s0, s1);
-      }
+      if (a.conv_tiled) circulant(A, B, reinterpret_cast<float *>(B + n), a.conv_h, n);
+      else circulant_long(A, B, a.conv_h, n);
       R = B;
     }
     __syncthreads();
@@ -689,15 +744,88 @@ template <int LAY> __device__ __forceinline__ int p2_soff(int off) {
   return LAY == LAY_PAD ? off + (off >> 4) : off;
 }
 
-// values per thread of the register-resident kernel for rows of n samples (0: none)
+// values per thread of the register-resident kernel for transforms of n samples (0: none)
 static int p2_values(int n) {
   switch (n) {
     case 256: case 512: return 8;
-    case 1024: case 2048: case 4096: return 16;
+    case 1024: case 2048: case 4096: case 8192: return 16;
     case 384: return 12;
-    case 768: case 1536: case 3072: return 24;
+    case 768: case 1536: case 3072: case 6144: return 24;
     default: return 0;
   }
+}
+
+// Rows of any other length n: R-weighting is a circular convolution with a real, even
+// kernel h, and a circular convolution of length n is part of one of length M >= 2n - 1
+// whose kernel is h at distances below n and 0 beyond -- real and even again, so it has a
+// real spectrum and the row kernel applies it like a table of weights, to rows padded with
+// zeros (FP32 staging).  717 rows x 77 views with the means: 1023 samples (3*11*31) 13.4 ms by
+// the O(n^2) convolution, 0.34 this way; 1000 samples (radix by radix) 0.79 and 0.34.  512 rows
+// x 61 views: 1440 samples 0.68 and 0.39, 192 samples 0.22 and 0.06.
+int p2_transform_length(int n) {
+  if (p2_values(n) && n <= 4096) return n;
+  for (int M : {256, 512, 768, 1024, 1536, 2048, 3072, 4096, 6144, 8192})
+    if (M >= 2 * n - 1) return M;
+  return 0;
+}
+
+namespace {
+using cplx = std::complex<double>;
+// Forward transform of x (length 2^k or 3*2^k), w = exp(-2 pi i j / size) of the top level
+void host_fft(cplx *x, cplx *tmp, int n, const cplx *w, int ws) {
+  if (n == 1) return;
+  const int R = n % 2 == 0 ? 2 : 3, m = n / R;
+  for (int r = 0; r < R; ++r)
+    for (int i = 0; i < m; ++i) tmp[r * m + i] = x[i * R + r];
+  for (int r = 0; r < R; ++r) host_fft(tmp + r * m, x + r * m, m, w, ws * R);
+  for (int k = 0; k < m; ++k) {
+    if (R == 2) {
+      const cplx a = tmp[k], b = tmp[m + k] * w[k * ws];
+      x[k] = a + b;
+      x[k + m] = a - b;
+    } else {
+      const cplx a = tmp[k], b = tmp[m + k] * w[k * ws], c = tmp[2 * m + k] * w[2 * k * ws];
+      const cplx s = b + c, d = cplx(0.0, -0.866025403784438646763723170752936183) * (b - c);
+      x[k] = a + s;
+      x[k + m] = a - 0.5 * s + d;
+      x[k + 2 * m] = a - 0.5 * s - d;
+    }
+  }
+}
+std::vector<cplx> roots(int n) {
+  std::vector<cplx> w(n);
+  for (int j = 0; j < n; ++j) w[j] = std::polar(1.0, -2.0 * M_PI * j / n);
+  return w;
+}
+}  // namespace
+
+// The weights of a padded transform of M samples for rows of n < M whose radial weights
+// are wt (real, wt[k] = wt[n - k]): the spectrum of the extended kernel, over M (the inverse's
+// scale).  The kernel h itself is wt's transform of length n, by Bluestein's chirp
+// convolution; all in double.
+void p2_padded_weights(int n, int M, const float *wt, float *out) {
+  int L = 1;
+  while (L < 2 * n - 1) L *= 2;
+  std::vector<cplx> a(L), b(L), tmp(std::max(L, M)), chirp(n);
+  const std::vector<cplx> wl = roots(L);
+  for (int k = 0; k < n; ++k) {
+    chirp[k] = std::polar(1.0, -M_PI * (double)((long long)k * k % (2LL * n)) / n);
+    a[k] = (double)wt[k] * chirp[k];
+    b[k] = std::conj(chirp[k]);
+    if (k) b[L - k] = b[k];
+  }
+  host_fft(a.data(), tmp.data(), L, wl.data(), 1);
+  host_fft(b.data(), tmp.data(), L, wl.data(), 1);
+  for (int i = 0; i < L; ++i) a[i] = std::conj(a[i] * b[i]);
+  host_fft(a.data(), tmp.data(), L, wl.data(), 1);
+  std::vector<cplx> h(M);
+  for (int m = 0; m < n; ++m) {
+    const double v = (std::conj(a[m]) * chirp[m]).real() / L / n;
+    h[m] = v;
+    if (m) h[M - m] = v;
+  }
+  host_fft(h.data(), tmp.data(), M, roots(M).data(), 1);
+  for (int k = 0; k < M; ++k) out[k] = (float)(h[k].real() / M);
 }
 
 bool p2_twiddle_table(int n, std::vector<float2> &out) {
@@ -841,37 +969,61 @@ __device__ __forceinline__ float2 *p2_inverse(float2 (&x)[V], int t, const float
   else return p2_inverse<N, V, I + 1>(x, t, tw, B, A);
 }
 
-template <int N, int V, int FMT, int STORE>
+// PAD: rows of n < N samples padded to the transform's N, weights of p2_padded_weights.
+// Their mean is taken off first: weight 0 is 0, so the result does not depend on it, and
+// the edges of the padded row would otherwise put its rounding into every sample.
+template <int N, int V, int FMT, int STORE, bool PAD>
 __device__ __forceinline__ void filter_p2_body(const FilterArgs &a, const int jp, const int v) {
   extern __shared__ __align__(16) unsigned char fsm[];
   constexpr int T = N / V;
+  const int n = PAD ? a.nx : N;  // samples of a row
   float2 *A = reinterpret_cast<float2 *>(fsm);
   float2 *B = A + padded_len<N>();
   const int t = threadIdx.x;
   const int r0 = 2 * jp;
   const bool has1 = r0 + 1 < a.ny;
-  const float *in0 = a.in + ((size_t)v * a.ny + r0) * N;
-  const float *sb0 = a.sub ? a.sub + ((size_t)v * a.ny + r0) * N : nullptr;
+  const float *in0 = a.in + ((size_t)v * a.ny + r0) * n;
+  const float *sb0 = a.sub ? a.sub + ((size_t)v * a.ny + r0) * n : nullptr;
   float2 x[V];
 #pragma unroll
   for (int j = 0; j < V; ++j) {
     const int k = t + j * T;
-    float x0 = __ldg(in0 + k), x1 = has1 ? __ldg(in0 + N + k) : 0.0f;
+    if (PAD && k >= n) {
+      x[j] = make_float2(0.0f, 0.0f);
+      continue;
+    }
+    float x0 = __ldg(in0 + k), x1 = has1 ? __ldg(in0 + n + k) : 0.0f;
     if (sb0) {  // SIRT residual: orig - reprojection (main.rs:933-935)
       x0 = __fsub_rn(x0, __ldg(sb0 + k));
-      if (has1) x1 = __fsub_rn(x1, __ldg(sb0 + N + k));
+      if (has1) x1 = __fsub_rn(x1, __ldg(sb0 + n + k));
     }
     x[j] = make_float2(x0, x1);
+  }
+  if (PAD) {
+    __shared__ float2 part[T / 32];
+    float2 s = make_float2(0.0f, 0.0f);
+#pragma unroll
+    for (int j = 0; j < V; ++j) s = cadd_p(s, x[j]);
+    for (int o = 16; o > 0; o >>= 1)
+      s = cadd_p(s, make_float2(__shfl_xor_sync(0xffffffffu, s.x, o), __shfl_xor_sync(0xffffffffu, s.y, o)));
+    if ((t & 31) == 0) part[t >> 5] = s;
+    __syncthreads();
+    s = part[0];
+    for (int w = 1; w < T / 32; ++w) s = cadd_p(s, part[w]);
+    const float2 mean = make_float2(__fdiv_rn(s.x, (float)n), __fdiv_rn(s.y, (float)n));
+#pragma unroll
+    for (int j = 0; j < V; ++j)
+      if (t + j * T < n) x[j] = csub_p(x[j], mean);
   }
   p2_forward<N, V, 0>(x, t, a.tw2, A, B);
   // x[j] = spectrum value t + j*T: x the radial weight, and for 2^k lengths the
   // 1/n of the inverse too (a power of two: exact, and exact through the
   // inverse's linear arithmetic, so the result is the one of scaling afterwards)
-  constexpr bool POW2 = (N & (N - 1)) == 0;
+  constexpr bool POW2 = PAD || (N & (N - 1)) == 0;  // padded: the weights hold the scale
 #pragma unroll
   for (int j = 0; j < V; ++j) {
     float w = __ldg(&a.weights[t + j * T]);
-    if (POW2) w = __fmul_rn(w, a.inv_n);
+    if (POW2 && !PAD) w = __fmul_rn(w, a.inv_n);
     x[j] = make_float2(__fmul_rn(x[j].x, w), __fmul_rn(x[j].y, w));
   }
   // the forward's last exchange read buffer A (odd pass count) or B; the
@@ -883,10 +1035,10 @@ __device__ __forceinline__ void filter_p2_body(const FilterArgs &a, const int jp
     const float2 z = Rr[k];  // plain layout
     return POW2 ? z : up2(mul2(pk2(z.x, z.y), pk2(inv_n, inv_n)));
   };
-  // final value of both rows at column k (0 <= k < N): the cosine stretch
+  // final value of both rows at column k (0 <= k < n): the cosine stretch
   // (main.rs:446-488) of the scaled inverse, or the scaled inverse itself
   const float stretch = a.stretch ? a.stretch[v] : 0.0f;
-  const float center = __fdiv_rn((float)N, 2.0f);
+  const float center = __fdiv_rn((float)n, 2.0f);
   auto fin = [&](int k) -> float2 {
     if (stretch == 0.0f) return sc(k);
     const float dx = __fsub_rn((float)k, center);
@@ -894,25 +1046,25 @@ __device__ __forceinline__ void filter_p2_body(const FilterArgs &a, const int jp
     const float fl = floorf(src_x);
     const int sx0 = fl < -1.0e9f ? -1000000000 : (int)fl;
     const float frac = __fsub_rn(src_x, fl);
-    if (a.cubic && sx0 >= 1 && sx0 + 2 < N) {
+    if (a.cubic && sx0 >= 1 && sx0 + 2 < n) {
       const float2 p0 = sc(sx0 - 1), p1 = sc(sx0), p2 = sc(sx0 + 1), p3 = sc(sx0 + 2);
       return make_float2(cubic1d(p0.x, p1.x, p2.x, p3.x, frac), cubic1d(p0.y, p1.y, p2.y, p3.y, frac));
     }
-    if (sx0 >= 0 && sx0 + 1 < N) {
+    if (sx0 >= 0 && sx0 + 1 < n) {
       const float2 p0 = sc(sx0), p1 = sc(sx0 + 1);
       const float omf = __fsub_rn(1.0f, frac);
       // RN(RN(p0*(1-f)) + RN(p1*f)) for both rows on the packed pipe (each lane is
       // the scalar operation: no product contracted into the sum)
       return up2(add2(mul2(pk2(p0.x, p0.y), pk2(omf, omf)), mul2(pk2(p1.x, p1.y), pk2(frac, frac))));
     }
-    if (sx0 >= 0 && sx0 < N) return sc(sx0);
+    if (sx0 >= 0 && sx0 < n) return sc(sx0);
     return make_float2(0.0f, 0.0f);
   };
   // pack into the staging format with the reference's fill rule (main.rs:386-406)
   const float fillv = a.fill ? a.fill[v] : 0.0f;
   auto fill = [&](int k) -> float2 {
     if (a.fill_mode == TG_FILL_ZERO) return make_float2(0.0f, 0.0f);
-    if (a.fill_mode == TG_FILL_EDGE) return fin(k < 0 ? 0 : N - 1);
+    if (a.fill_mode == TG_FILL_EDGE) return fin(k < 0 ? 0 : n - 1);
     return make_float2(fillv, fillv);
   };
   float hmax = 0.0f;  // largest |value| packed into FP16 by this thread
@@ -920,7 +1072,7 @@ __device__ __forceinline__ void filter_p2_body(const FilterArgs &a, const int jp
     OctWriter ow(a, v, jp);
     for (int e = t; e < a.PW; e += T) {
       const int k = e - a.padL;
-      float2 z = k >= 0 && k < N ? fin(k) : fill(k);
+      float2 z = k >= 0 && k < n ? fin(k) : fill(k);
       if (!has1) z.y = 0.0f;
       ow.put(e, z.x, z.y);
     }
@@ -937,10 +1089,10 @@ __device__ __forceinline__ void filter_p2_body(const FilterArgs &a, const int jp
     const int e = e0 + lane;
     const int k = e - a.padL;
     float2 lo = make_float2(0.0f, 0.0f);
-    if (k >= 0 && k < N) lo = fin(k);
+    if (k >= 0 && k < n) lo = fin(k);
     float2 hi = make_float2(__shfl_down_sync(0xffffffffu, lo.x, 1), __shfl_down_sync(0xffffffffu, lo.y, 1));
     if (lane == 31 || e >= a.PW) continue;
-    if (!(k >= 0 && k + 1 < N)) lo = hi = fill(k);
+    if (!(k >= 0 && k + 1 < n)) lo = hi = fill(k);
     if (!has1) lo.y = hi.y = 0.0f;
     if (FMT == FMT_ROWPAIR) {
       uint8_t *out = reinterpret_cast<uint8_t *>(a.out) +
@@ -979,11 +1131,11 @@ __device__ __forceinline__ void filter_p2_body(const FilterArgs &a, const int jp
 // 4 of 256 threads for the radix-8 kernels; 5 of the radix-16 kernels' 64 or 128
 // threads (96 registers, no spills at 2048), 2 of 256
 __host__ __device__ constexpr int p2_min_blocks(int N, int V) {
-  return V == 8 && N / V == 256 ? 4 : V == 16 ? (N / V == 256 ? 2 : 5) : 1;
+  return V == 8 && N / V == 256 ? 4 : V == 16 ? (N / V == 512 ? 1 : N / V == 256 ? 2 : 5) : 1;
 }
-template <int N, int V, int FMT, int STORE>
+template <int N, int V, int FMT, int STORE, bool PAD>
 __global__ void __launch_bounds__(N / V, p2_min_blocks(N, V)) filter_p2_kernel(FilterArgs a) {
-  filter_p2_body<N, V, FMT, STORE>(a, blockIdx.x, blockIdx.y);
+  filter_p2_body<N, V, FMT, STORE, PAD>(a, blockIdx.x, blockIdx.y);
 }
 
 // The same filter over the row pairs of many series of one width: block b
@@ -1009,42 +1161,72 @@ __global__ void __launch_bounds__(N / V, p2_min_blocks(N, V)) filter_p2_batch_ke
   for (int i = threadIdx.x; i < (int)(sizeof(FilterArgs) / 4); i += blockDim.x) dst[i] = src[i];
   __syncthreads();
   const int t = (int)blockIdx.x - __ldg(&fb.blk0[j]), nrp = (s_a.ny + 1) / 2;
-  filter_p2_body<N, V, FMT, STORE>(s_a, t % nrp, t / nrp);
+  filter_p2_body<N, V, FMT, STORE, false>(s_a, t % nrp, t / nrp);
 }
 
-template <int N, int V, int FMT, int STORE> static void launch_p2(const FilterArgs &a, cudaStream_t st) {
+template <int N, int V, int FMT, int STORE, bool PAD> static void launch_p2(const FilterArgs &a, cudaStream_t st) {
   const size_t smem = (size_t)padded_len<N>() * 16;
-  auto k = filter_p2_kernel<N, V, FMT, STORE>;
+  auto k = filter_p2_kernel<N, V, FMT, STORE, PAD>;
   if (smem > 48 * 1024) cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   k<<<dim3((a.ny + 1) / 2, a.nviews), N / V, smem, st>>>(a);
 }
 
 template <int FMT, int STORE> static bool try_p2(const FilterArgs &a, cudaStream_t st) {
-  if (!a.weights || a.conv_h || !a.tw2 || getenv("TG_FILTER_GENERIC")) return false;
-  switch (a.nx) {
-    case 256: launch_p2<256, 8, FMT, STORE>(a, st); return true;
-    case 512: launch_p2<512, 8, FMT, STORE>(a, st); return true;
-    case 1024: launch_p2<1024, 16, FMT, STORE>(a, st); return true;
-    case 2048: launch_p2<2048, 16, FMT, STORE>(a, st); return true;
-    case 4096: launch_p2<4096, 16, FMT, STORE>(a, st); return true;
-    case 384: launch_p2<384, 12, FMT, STORE>(a, st); return true;  // 3 * 2^k: 12 or 24 values per thread
-    case 768: launch_p2<768, 24, FMT, STORE>(a, st); return true;
-    case 1536: launch_p2<1536, 24, FMT, STORE>(a, st); return true;
-    case 3072: launch_p2<3072, 24, FMT, STORE>(a, st); return true;
+  if (!a.weights || !a.fft_n) return false;
+#define TG_P2(N, V, PAD) \
+  case N: launch_p2<N, V, FMT, STORE, PAD>(a, st); return true;
+  if (a.fft_n == a.nx) switch (a.nx) {
+      TG_P2(256, 8, false)
+      TG_P2(512, 8, false)
+      TG_P2(1024, 16, false)
+      TG_P2(2048, 16, false)
+      TG_P2(4096, 16, false)
+      TG_P2(384, 12, false)  // 3 * 2^k: 12 or 24 values per thread
+      TG_P2(768, 24, false)
+      TG_P2(1536, 24, false)
+      TG_P2(3072, 24, false)
+      default: return false;
+    }
+  switch (a.fft_n) {
+    TG_P2(256, 8, true)
+    TG_P2(512, 8, true)
+    TG_P2(768, 24, true)
+    TG_P2(1024, 16, true)
+    TG_P2(1536, 24, true)
+    TG_P2(2048, 16, true)
+    TG_P2(3072, 24, true)
+    TG_P2(4096, 16, true)
+    TG_P2(6144, 24, true)
+    TG_P2(8192, 16, true)
     default: return false;
   }
+#undef TG_P2
 }
 
-template <int FMT, int STORE> static void launch_f(const FilterArgs &a, cudaStream_t st) {
-  if (try_p2<FMT, STORE>(a, st)) return;
-  size_t smem = (size_t)a.nx * 16;  // two complex ping-pong buffers
+// threads and shared memory of the generic kernel: two complex ping-pong buffers, and for
+// the convolution its taps and one thread per CONV_R outputs
+static int generic_shape(FilterArgs &a, size_t *smem) {
+  *smem = (size_t)a.nx * 16;
+  if (!a.weights || !a.conv_h) return 256;
+  a.conv_tiled = conv_tiled(a.nx);
+  if (!a.conv_tiled) return 256;
+  *smem += 4 * CONV_R * (size_t)conv_cols(a.nx);
+  const int passes = (a.nx + CONV_R * 256 - 1) / (CONV_R * 256);
+  return ((a.nx + CONV_R * passes - 1) / (CONV_R * passes) + 31) & ~31;
+}
+
+template <int FMT, int STORE> static void launch_f(const FilterArgs &a0, cudaStream_t st) {
+  if (try_p2<FMT, STORE>(a0, st)) return;
+  FilterArgs a = a0;
+  size_t smem;
+  const int threads = generic_shape(a, &smem);
   auto k = filter_kernel<FMT, STORE>;
   if (smem > 48 * 1024) cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  k<<<dim3((a.ny + 1) / 2, a.nviews), 256, smem, st>>>(a);
+  k<<<dim3((a.ny + 1) / 2, a.nviews), threads, smem, st>>>(a);
 }
 
 int filter_batch_width(const FilterArgs &a) {
-  if (!a.weights || a.conv_h || !a.tw2 || getenv("TG_FILTER_GENERIC")) return 0;
+  if (!a.weights || a.fft_n != a.nx) return 0;
   switch (a.nx) {
     case 256: case 512: case 1024: case 2048: case 4096: case 384: case 768: case 1536: case 3072: return a.nx;
     default: return 0;
@@ -1245,14 +1427,15 @@ extern "C" int tg_apply_rweighting_device_noalloc(float *dev_proj, size_t in_nx,
   f.fmt = FMT_ROWS;
   f.store = TG_STORE_FP32;
   f.inv_n = 1.0f / (float)n;
-  size_t smem = (size_t)n * 16;
+  size_t smem;
+  const int threads = generic_shape(f, &smem);
   auto k = filter_kernel<FMT_ROWS, TG_STORE_FP32>;
   if (smem > 48 * 1024 &&
       (e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) != cudaSuccess) {
     restore();
     return cuda_fail(e, "cudaFuncSetAttribute(filter)");
   }
-  k<<<dim3((unsigned)((in_ny + 1) / 2), (unsigned)nz), 256, smem, st>>>(f);
+  k<<<dim3((unsigned)((in_ny + 1) / 2), (unsigned)nz), threads, smem, st>>>(f);
   e = cudaGetLastError();
   restore();
   if (e != cudaSuccess) return cuda_fail(e, "filter launch (noalloc)");

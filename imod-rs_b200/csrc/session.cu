@@ -299,7 +299,8 @@ FilterArgs filter_args(tg_session *s, bool residual) {
   f.out = s->d_pairs;
   f.weights = s->o.no_weight ? nullptr : s->d_weights;
   f.tw = s->d_tw;
-  f.tw2 = s->has_tw2 ? s->d_tw + s->nx : nullptr;
+  f.fft_n = s->fft_n;
+  f.tw2 = s->fft_n ? s->d_tw + s->nx : nullptr;
   f.conv_h = s->use_conv ? s->d_conv : nullptr;
   f.stretch = residual ? nullptr : s->d_stretch;
   f.fill = s->d_means;
@@ -676,8 +677,12 @@ int tg::session_create_ex(const tg_geometry *g, const tg_options *opt, cudaMemPo
                   : s->fmt == FMT_OCT   ? (s->ny + 15) / 16 * 2
                                         : s->ny;
 
-  // FFT plan or circulant fallback
-  s->use_conv = !fft_plan(s->nx, &s->plan);
+  // transform of the register-resident filter kernel, else an FFT plan, else circulant
+  s->fft_n = opt->no_weight || getenv("TG_FILTER_GENERIC") ? 0 : p2_transform_length(s->nx);
+  // half staging rounds the filtered samples, so there another transform of a row (equal to
+  // 1e-6) would move every rounding decision near a midpoint: only the row's own length
+  if (s->store != TG_STORE_FP32 && s->fft_n != s->nx) s->fft_n = 0;
+  s->use_conv = !fft_plan(s->nx, &s->plan) && !s->fft_n;
   if (s->nx * 16 > 200 * 1024) { set_error("rows wider than 12800 are not supported"); return fail(TG_ERR_UNSUPPORTED); }
 
   cudaError_t ce = cudaSuccess;
@@ -709,7 +714,8 @@ int tg::session_create_ex(const tg_geometry *g, const tg_options *opt, cudaMemPo
       (rc = dalloc(s, &s->d_part, (size_t)s->ny * ntiles * sizeof(StatPartial))) ||
       (rc = dalloc(s, &s->d_slice_stats, (size_t)s->ny * 12)) || (rc = dalloc(s, &s->d_stats3, 16)) ||
       (rc = dalloc(s, &s->d_vg, (size_t)s->nviews * 16)) || (rc = dalloc(s, &s->d_vg2, (size_t)s->nviews * 16)) ||
-      (rc = dalloc(s, &s->d_weights, (size_t)s->nx * 4)) || (rc = dalloc(s, &s->d_tw, (size_t)s->nx * 16)) ||
+      (rc = dalloc(s, &s->d_weights, (size_t)std::max(s->nx, s->fft_n) * 4)) ||
+      (rc = dalloc(s, &s->d_tw, ((size_t)s->nx + std::max(s->nx, s->fft_n)) * 8)) ||
       (rc = dalloc(s, &s->d_stretch, (size_t)s->nviews * 4)) || (rc = dalloc(s, &s->d_err, 16)))
     return fail(rc);
   if (s->mma_steps && (rc = dalloc(s, &s->d_tmap, 128))) return fail(rc);
@@ -761,14 +767,14 @@ int tg::session_create_ex(const tg_geometry *g, const tg_options *opt, cudaMemPo
 
   std::vector<float> wt(s->nx);
   weight_table(s->nx, opt->radial_cutoff, opt->radial_falloff, opt->exact_filter_size, opt->hamming, wt.data());
-  // [0, nx): exp(-2 pi i k/nx); [nx, 2 nx - 1): the register-resident kernel's
+  // [0, nx): exp(-2 pi i k/nx); from nx: the register-resident kernel's
   // per-pass table, for the widths that have that kernel
-  std::vector<float2> tw(2 * (size_t)s->nx, make_float2(0.0f, 0.0f)), tw2;
+  std::vector<float2> tw((size_t)s->nx + std::max(s->nx, s->fft_n), make_float2(0.0f, 0.0f)), tw2;
   for (int k = 0; k < s->nx; ++k) {
     double a = -2.0 * M_PI * (double)k / (double)s->nx;
     tw[k] = make_float2((float)cos(a), (float)sin(a));
   }
-  s->has_tw2 = p2_twiddle_table(s->nx, tw2);
+  if (s->fft_n) p2_twiddle_table(s->fft_n, tw2);
   std::copy(tw2.begin(), tw2.end(), tw.begin() + s->nx);
   if (s->use_conv) {
     // h[m] = (1/n) * sum_k w[k] exp(2 pi i k m / n)  (w real and even)
@@ -786,6 +792,11 @@ int tg::session_create_ex(const tg_geometry *g, const tg_options *opt, cudaMemPo
     double w2 = 0.0;
     for (float w : wt) w2 += (double)w * w;
     s->oct_gain = (float)std::max(1.0, sqrt(w2)) * (opt->cosine_cubic ? 1.25f : 1.0f);
+  }
+  if (s->fft_n > s->nx) {
+    std::vector<float> padded(s->fft_n);
+    p2_padded_weights(s->nx, s->fft_n, wt.data(), padded.data());
+    wt.swap(padded);
   }
   // on the session's stream (after its stream-ordered allocations); pageable
   // sources have been staged when each call returns; synchronised below

@@ -80,10 +80,12 @@ struct FilterArgs {
   const float *in;          // [nviews_all][ny][nx]
   const float *sub;         // optional: value = in - sub (SIRT residual)
   void *out;                // staged format
-  const float *weights;     // n weights, nullptr = no R-weighting
+  const float *weights;     // fft_n (else nx) weights, nullptr = no R-weighting
   const float2 *tw;         // n twiddles exp(-2 pi i k/n)
   const float2 *tw2;        // register-resident kernel's per-pass twiddles (p2_twiddle_table), or nullptr
+  int fft_n;                // transform of the register-resident kernel (p2_transform_length), 0: generic kernel
   const float *conv_h;      // circulant kernel for n without a radix plan (else nullptr)
+  int conv_tiled;           // set by the launcher: its taps fit in shared memory
   const float *stretch;     // per view 1/cos (f32) or 0: no stretch; nullptr = none
   const float *fill;        // per view fill value for mean mode
   int nx, ny, nviews;
@@ -103,6 +105,11 @@ void launch_filter(const FilterArgs &a, cudaStream_t st);
 // offset_p + (r-1)*NS + k (k-major, so a warp's lanes read neighbouring entries);
 // fewer than n entries in all.  False (table empty) when n has no such kernel.
 bool p2_twiddle_table(int n, std::vector<float2> &out);
+// Length of the register-resident kernel's transform for rows of n samples: n itself (2^k,
+// 3*2^k), a padded length, or 0 (rows beyond 4096 samples: generic kernel); and the weights
+// of a padded one from the rows' n
+int p2_transform_length(int n);
+void p2_padded_weights(int n, int M, const float *wt, float *out);
 // ---- the register-resident filter over many series of one width in one launch ----
 struct FilterBatchDev {
   const FilterArgs *jobs;   // device array
