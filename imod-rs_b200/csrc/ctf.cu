@@ -29,7 +29,8 @@
 // 512x512x41 with 16-pixel strips (1312 strips), host to host: 88.7 ms with nine
 // launches per strip (11,852 launches, bound by the launching thread and by
 // grids of a few blocks), 18.0 ms batched, of which the copies from and to the
-// caller's pageable memory take about 12.
+// caller's pageable memory take about 12 (about 13 in all with the output pages
+// faulted in meanwhile, fault_ahead.h).
 //
 // Layout in device memory: the stack [nz][ny][nx] f32, corrected in place; two
 // buffers of a chunk's strips (sw*sh float2 each); the strip and view tables;
@@ -44,6 +45,7 @@
 #include <string>
 #include <vector>
 
+#include "fault_ahead.h"
 #include "fft.cuh"
 #include "tg_internal.h"
 
@@ -538,6 +540,7 @@ int tg_ctf_phaseflip(const tg_ctf_options *o, const float *host_in, int32_t nx, 
   TG_CUDA(cudaStreamCreateWithFlags(&mem.st, cudaStreamNonBlocking));
   cudaStream_t st = mem.st;
   const size_t npix = (size_t)nx * ny, ntot = npix * nz;
+  FaultAhead out_pages(host_out, ntot * 4);
   // Views per chunk, or (0) runs of strips of one view: whole views where they fit.
   const size_t view_bytes = std::max<size_t>(view_samples, 1) * 2 * sizeof(float2);
   int nv = kept > 0 && kept <= 65535 ? (int)std::min<size_t>({CTF_CHUNK_BYTES / view_bytes, (size_t)(65535 / kept), (size_t)nz}) : 0;
@@ -667,6 +670,7 @@ int tg_ctf_phaseflip(const tg_ctf_options *o, const float *host_in, int32_t nx, 
     launch_stats_reduce(d_part, nz, ntiles, (int)npix, d_slice, d_stats3, st);
     TG_CUDA(cudaGetLastError());
   }
+  out_pages.join();
   TG_CUDA(cudaMemcpyAsync(host_out, d_stack, ntot * 4, cudaMemcpyDeviceToHost, st));
   float s3[3];
   TG_CUDA(cudaMemcpyAsync(s3, d_stats3, 12, cudaMemcpyDeviceToHost, st));

@@ -21,6 +21,7 @@
 #include <tuple>
 #include <vector>
 
+#include "fault_ahead.h"
 #include "session_impl.h"
 
 namespace tg {
@@ -1027,9 +1028,11 @@ int tg_synchronize(tg_session *s) {
 
 int tg_download_slices(tg_session *s, int32_t y0, int32_t y1, float *host_out, tg_stats *stats) {
   if (!s || y0 < 0 || y1 > s->ny || y0 > y1 || (!host_out && y1 > y0)) return TG_ERR_INVALID_ARG;
+  size_t sl = (size_t)s->onx * s->onz;
+  FaultAhead out_pages(host_out, (size_t)(y1 - y0) * sl * 4);
   int rc = tg_synchronize(s);
   if (rc != TG_OK) return rc;
-  size_t sl = (size_t)s->onx * s->onz;
+  out_pages.join();
   if (y1 > y0)
     TG_CUDA(cudaMemcpyAsync(host_out, s->d_vol + (size_t)y0 * sl, (size_t)(y1 - y0) * sl * 4,
                             cudaMemcpyDeviceToHost, s->st));
