@@ -136,24 +136,45 @@ __global__ void __launch_bounds__(256) slice_stats_kernel(const StatPartial *par
   }
 }
 
-__global__ void fold_slices_kernel(const float *slice_stats, int ny, int count, float *out3) {
+// The fold is a serial chain in Y order.  The block fetches the slices' statistics
+// and forms the products, one thread chains them out of shared memory; with that
+// thread also loading them the kernel waited for memory slice by slice (512
+// slices: 25.8 us, now 6).
+constexpr int FOLD_SLICES = 1024;
+__global__ void __launch_bounds__(256) fold_slices_kernel(const float *slice_stats, int ny, int count, float *out3) {
+  __shared__ float2 mm[FOLD_SLICES];
+  __shared__ double part[FOLD_SLICES];
   float gmin = 3.40282347e+38f, gmax = -3.40282347e+38f;
   double gsum = 0.0;
-  for (int iy = 0; iy < ny; ++iy) {
-    const float smin = slice_stats[3 * iy], smax = slice_stats[3 * iy + 1], smean = slice_stats[3 * iy + 2];
-    if (smin < gmin) gmin = smin;
-    if (smax > gmax) gmax = smax;
-    gsum += (double)smean * (double)count;
+  for (int y0 = 0; y0 < ny; y0 += FOLD_SLICES) {
+    const int n = min(FOLD_SLICES, ny - y0);
+    __syncthreads();
+    for (int i = threadIdx.x; i < n; i += blockDim.x) {
+      const float *p = slice_stats + 3 * (size_t)(y0 + i);
+      mm[i] = make_float2(p[0], p[1]);
+      part[i] = (double)p[2] * (double)count;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+#pragma unroll 8
+      for (int i = 0; i < n; ++i) {
+        if (mm[i].x < gmin) gmin = mm[i].x;
+        if (mm[i].y > gmax) gmax = mm[i].y;
+        gsum += part[i];
+      }
+    }
   }
-  out3[0] = gmin;
-  out3[1] = gmax;
-  out3[2] = (float)(gsum / ((double)count * (double)ny));
+  if (threadIdx.x == 0) {
+    out3[0] = gmin;
+    out3[1] = gmax;
+    out3[2] = (float)(gsum / ((double)count * (double)ny));
+  }
 }
 
 void launch_stats_reduce(const StatPartial *partial, int ny, int ntiles, int count,
                          float *slice_stats, float *out3, cudaStream_t st) {
   slice_stats_kernel<<<ny, 256, 0, st>>>(partial, ntiles, count, slice_stats);
-  fold_slices_kernel<<<1, 1, 0, st>>>(slice_stats, ny, count, out3);
+  fold_slices_kernel<<<1, 256, 0, st>>>(slice_stats, ny, count, out3);
 }
 
 // f32 -> IEEE half, round to nearest even, for mode-12 output (n values).  With
