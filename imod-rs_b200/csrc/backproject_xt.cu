@@ -332,48 +332,43 @@ __global__ void __launch_bounds__(256) xt_blend_kernel(BpArgs a, const float *__
     const float w0 = __fsub_rn(1.0f, fr);
     const float *b0 = rows + ((two || one) ? (size_t)sy0 * sl : 0) + ox;
     float *out = a.vol + (size_t)iy * sl + ox;
-    auto blend = [&](size_t o) {
-      float v = 0.0f;
-      if (two) v = __fadd_rn(__fmul_rn(__ldg(b0 + o), w0), __fmul_rn(__ldg(b0 + sl + o), fr));
-      else if (one) v = __ldg(b0 + o);
-      return v;
-    };
-    if (MODE == 2) {
-      // vol += relax * v, four depths at a time: their old values are loaded
-      // before any of their stores (a store through out could alias a later
-      // load as far as the compiler knows, so one update at a time would wait
-      // for each load's round trip to HBM in turn)
-      int oz = oz0;
-      for (; oz + 4 <= oz1; oz += 4) {
-        float old[4];
+    // N depths at a time, all their loads before any store (a store through out could
+    // alias a later load as far as the compiler knows, and each update would wait for
+    // its own round trip to HBM).  1024x1024x400, update: 4 depths with the rows' loads
+    // behind the stores 1.30 ms, 8 depths with all loads ahead 0.99 (5.0 GB); the raw
+    // sums of mode 1 0.94 -> 0.63 (3.4 GB)
+    auto depths = [&](int oz, auto nc) {
+      constexpr int N = decltype(nc)::value;
+      float old[N], p[N], q[N];
 #pragma unroll
-        for (int u = 0; u < 4; ++u) old[u] = out[(size_t)(oz + u) * a.onx];
+      for (int u = 0; u < N; ++u) {
+        const size_t o = (size_t)(oz + u) * a.onx;
+        old[u] = MODE == 2 ? __ldcs(out + o) : 0.0f;
+        p[u] = two || one ? __ldg(b0 + o) : 0.0f;
+        q[u] = two ? __ldg(b0 + sl + o) : 0.0f;
+      }
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          const size_t o = (size_t)(oz + u) * a.onx;
-          out[o] = __fadd_rn(old[u], __fmul_rn(a.relax, blend(o)));
+      for (int u = 0; u < N; ++u) {
+        const float v = two ? __fadd_rn(__fmul_rn(p[u], w0), __fmul_rn(q[u], fr)) : p[u];
+        float y = v;  // MODE 1
+        if (MODE == 0) {
+          y = __fadd_rn(__fmul_rn(__fmul_rn(v, a.dw), a.os), a.oa);
+          mn = fminf(mn, y);
+          mx = fmaxf(mx, y);
+          sum += (double)y;
+        } else if (MODE == 2) {
+          y = __fadd_rn(old[u], __fmul_rn(a.relax, v));
         }
+        __stcs(out + (size_t)(oz + u) * a.onx, y);
       }
-      for (; oz < oz1; ++oz) {
-        const size_t o = (size_t)oz * a.onx;
-        out[o] = __fadd_rn(out[o], __fmul_rn(a.relax, blend(o)));
-      }
-      continue;
+    };
+    int oz = oz0;
+    for (; oz + 8 <= oz1; oz += 8) depths(oz, std::integral_constant<int, 8>{});
+    if (oz + 4 <= oz1) {
+      depths(oz, std::integral_constant<int, 4>{});
+      oz += 4;
     }
-#pragma unroll 4
-    for (int oz = oz0; oz < oz1; ++oz) {
-      const size_t o = (size_t)oz * a.onx;
-      const float v = blend(o);
-      if (MODE == 0) {
-        const float y = __fadd_rn(__fmul_rn(__fmul_rn(v, a.dw), a.os), a.oa);
-        out[o] = y;
-        mn = fminf(mn, y);
-        mx = fmaxf(mx, y);
-        sum += (double)y;
-      } else {  // MODE 1
-        out[o] = v;
-      }
-    }
+    for (; oz < oz1; ++oz) depths(oz, std::integral_constant<int, 1>{});
   }
   if (MODE == 0) {
     __shared__ float rmn[8], rmx[8];
