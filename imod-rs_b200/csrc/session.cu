@@ -1005,9 +1005,9 @@ int tg_sirt_restore(tg_session *s, const float *host_volume, int32_t iterations_
 int tg_synchronize(tg_session *s) {
   if (!s) return TG_ERR_INVALID_ARG;
   TG_CUDA(cudaSetDevice(s->dev));
+  int err[4] = {0, 0, 0, 0};  // the copy waits for the run: one wait, not one for each
+  TG_CUDA(cudaMemcpyAsync(err, s->d_err, 16, cudaMemcpyDeviceToHost, s->st));
   TG_CUDA(cudaStreamSynchronize(s->st));
-  int err[4] = {0, 0, 0, 0};
-  TG_CUDA(cudaMemcpy(err, s->d_err, 16, cudaMemcpyDeviceToHost));
   if (err[0]) {
     cudaMemsetAsync(s->d_err, 0, 16, s->st);
     return device_error_status(err[0]);
