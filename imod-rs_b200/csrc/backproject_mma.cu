@@ -251,7 +251,7 @@ __device__ __forceinline__ void mma_body(const Job &job, int ntiles, unsigned ch
         bool go = true;
         for (int i = 0; 2 * i < nviews; ++i) {
           const int e = i & 1;
-          if (!wait_phase(smem_u32(&tfull[e]), (ph >> e) & 1, &s_abort, limit)) {
+          if (!poll_phase(smem_u32(&tfull[e]), (ph >> e) & 1, &s_abort, limit)) {
             go = false;
             break;
           }
@@ -440,7 +440,7 @@ __device__ __forceinline__ void mma_body(const Job &job, int ntiles, unsigned ch
         g0 = __ldg(vg + min(v + 2, nviews - 1));
         g1 = __ldg(vg + min(v + 3, nviews - 1));
         const bool two = v + 1 < nviews;
-        if (!wait_phase(smem_u32(&empty[b]), ph, &s_abort, limit)) {
+        if (!poll_phase(smem_u32(&empty[b]), ph, &s_abort, limit)) {
           go = false;
           break;
         }
@@ -449,7 +449,7 @@ __device__ __forceinline__ void mma_body(const Job &job, int ntiles, unsigned ch
         if (two) store_row(wb, dst + C::VIEW);
         fence_proxy_async();
         // the first weight warp also waits for the windows, so that the issuing threads wait once
-        if (warp == NCONS && !wait_phase(smem_u32(&fullb[b]), ph ^ 1, &s_abort, limit)) {
+        if (warp == NCONS && !poll_phase(smem_u32(&fullb[b]), ph ^ 1, &s_abort, limit)) {
           go = false;
           break;
         }
@@ -485,7 +485,7 @@ __device__ __forceinline__ void mma_body(const Job &job, int ntiles, unsigned ch
           if ((v & 31) == 0) k0s = window_start<KW>(a, q, v + lane);
           const int ka = __shfl_sync(0xffffffffu, k0s, v & 31), kb = __shfl_sync(0xffffffffu, k0s, (v + 1) & 31);
           const bool two = v + 1 < nviews;
-          go = wait_phase(smem_u32(&empty[b]), ph, &s_abort, limit);
+          go = poll_phase(smem_u32(&empty[b]), ph, &s_abort, limit);
           go = __all_sync(0xffffffffu, go && !s_abort);  // one decision for the warp
           if (!go) break;
           if (v / 2 == skip) {  // test hook: no copy, fullb[b] never completes
@@ -509,7 +509,7 @@ __device__ __forceinline__ void mma_body(const Job &job, int ntiles, unsigned ch
       }
       if (s_abort && lane == 0)  // no copy may land after the CTA exits
         for (int g = max(0, issued - NST); g < issued; ++g)
-          if (g != skipped) wait_phase(smem_u32(&fullb[g % NST]), (g / NST) & 1, nullptr, limit);
+          if (g != skipped) poll_phase(smem_u32(&fullb[g % NST]), (g / NST) & 1, nullptr, limit);
     } else if (warp <= 14 && lane == 0) {
       // ---------------- tensor cores: one thread per tensor-memory buffer issues alternate
       // pairs of views ----------------
@@ -534,8 +534,8 @@ __device__ __forceinline__ void mma_body(const Job &job, int ntiles, unsigned ch
         advance(b, ph, e);
         for (int i = e; i < npairs; i += 2) {
           const bool two = 2 * i + 1 < nviews;
-          if (!wait_phase(smem_u32(&full[b]), ph, &s_abort, limit) ||
-              !wait_phase(smem_u32(&tempty[e]), tph, &s_abort, limit)) {
+          if (!poll_phase(smem_u32(&full[b]), ph, &s_abort, limit) ||
+              !poll_phase(smem_u32(&tempty[e]), tph, &s_abort, limit)) {
             go = false;
             break;
           }
@@ -568,7 +568,7 @@ __device__ __forceinline__ void mma_body(const Job &job, int ntiles, unsigned ch
       }
       if (!go) s_abort = 1;
       mma_commit(smem_u32(&done[e]));  // nothing in flight at exit
-      wait_phase(smem_u32(&done[e]), 0, nullptr, limit);
+      poll_phase(smem_u32(&done[e]), 0, nullptr, limit);
     }
   }
   __syncwarp();

@@ -121,7 +121,7 @@ __device__ __forceinline__ void raise_range(float mx, unsigned *range) {
   if ((threadIdx.x & 31) == 0 && m) atomicMax(range, m);
 }
 
-template <bool LOG>
+template <bool LOG, bool RANGE>
 __global__ void __launch_bounds__(256) log_sum_kernel(const float *__restrict__ raw, float *__restrict__ logd,
                                                       long npix, double *partials, unsigned *range) {
   const int v = blockIdx.y, c = blockIdx.x;
@@ -139,7 +139,7 @@ __global__ void __launch_bounds__(256) log_sum_kernel(const float *__restrict__ 
     float x = raw[base + i];
     if (LOG) logd[base + i] = x = log_sample_fast(x, lt);
     s += (double)x;
-    mx = fmaxf(mx, finite_abs(x));
+    if (RANGE) mx = fmaxf(mx, finite_abs(x));
   }
   const float4 *r4 = reinterpret_cast<const float4 *>(raw + base + a0);
   float4 *l4 = LOG ? reinterpret_cast<float4 *>(logd + base + a0) : nullptr;
@@ -155,21 +155,21 @@ __global__ void __launch_bounds__(256) log_sum_kernel(const float *__restrict__ 
     }
     s += ((double)x.x + (double)x.y) + ((double)x.z + (double)x.w);
     s += ((double)y.x + (double)y.y) + ((double)y.z + (double)y.w);
-    mx = fmaxf(mx, fmaxf(finite_abs4(x), finite_abs4(y)));
+    if (RANGE) mx = fmaxf(mx, fmaxf(finite_abs4(x), finite_abs4(y)));
   }
   if (i < n4) {
     const float4 x = log4<LOG>(__ldcs(r4 + i), lt);
     if (LOG) l4[i] = x;
     s += ((double)x.x + (double)x.y) + ((double)x.z + (double)x.w);
-    mx = fmaxf(mx, finite_abs4(x));
+    if (RANGE) mx = fmaxf(mx, finite_abs4(x));
   }
   for (long k = a1 + threadIdx.x; k < c1; k += blockDim.x) {
     float x = raw[base + k];
     if (LOG) logd[base + k] = x = log_sample_fast(x, lt);
     s += (double)x;
-    mx = fmaxf(mx, finite_abs(x));
+    if (RANGE) mx = fmaxf(mx, finite_abs(x));
   }
-  if (range) raise_range(mx, range);
+  if (RANGE) raise_range(mx, range);
   __shared__ double red[8];
   for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
   if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
@@ -222,8 +222,9 @@ __global__ void view_sums_kernel(const double *partials, int nviews, double *sum
 
 void launch_log_means(const float *raw, float *logd, int npix, int nviews, double *partials,
                       float *means, unsigned *range, cudaStream_t st) {
-  if (logd) log_sum_kernel<true><<<dim3(MEAN_CH, nviews), 256, 0, st>>>(raw, logd, npix, partials, range);
-  else log_sum_kernel<false><<<dim3(MEAN_CH, nviews), 256, 0, st>>>(raw, nullptr, npix, partials, range);
+  const dim3 grid(MEAN_CH, nviews);
+  if (logd) (range ? log_sum_kernel<true, true> : log_sum_kernel<true, false>)<<<grid, 256, 0, st>>>(raw, logd, npix, partials, range);
+  else (range ? log_sum_kernel<false, true> : log_sum_kernel<false, false>)<<<grid, 256, 0, st>>>(raw, nullptr, npix, partials, range);
   if (means) means_final_kernel<<<(nviews + 127) / 128, 128, 0, st>>>(partials, npix, nviews, means);
 }
 
