@@ -760,9 +760,11 @@ static int p2_values(int n) {
 // kernel h, and a circular convolution of length n is part of one of length M >= 2n - 1
 // whose kernel is h at distances below n and 0 beyond -- real and even again, so it has a
 // real spectrum and the row kernel applies it like a table of weights, to rows padded with
-// zeros (FP32 staging).  717 rows x 77 views with the means: 1023 samples (3*11*31) 13.4 ms by
-// the O(n^2) convolution, 0.34 this way; 1000 samples (radix by radix) 0.79 and 0.34.  512 rows
-// x 61 views: 1440 samples 0.68 and 0.39, 192 samples 0.22 and 0.06.
+// zeros.  Only tg_apply_rweighting takes it (FP32 SINGLE rows): it is nearer to 64 bits than
+// the convolution (1023 samples with a large mean: 1.3e-7 against 2.4e-6 relative), whose f32
+// taps do not sum to zero and leave a trace of a row's mean; but in a reconstruction that
+// difference moves the volume's mean by 4e-5 to 7e-2 of itself, and so sessions keep the
+// convolution or the radix-by-radix transform.
 int p2_transform_length(int n) {
   if (p2_values(n) && n <= 4096) return n;
   for (int M : {256, 512, 768, 1024, 1536, 2048, 3072, 4096, 6144, 8192})
@@ -1188,20 +1190,20 @@ template <int FMT, int STORE> static bool try_p2(const FilterArgs &a, cudaStream
       TG_P2(3072, 24, false)
       default: return false;
     }
-  switch (a.fft_n) {
-    TG_P2(256, 8, true)
-    TG_P2(512, 8, true)
-    TG_P2(768, 24, true)
-    TG_P2(1024, 16, true)
-    TG_P2(1536, 24, true)
-    TG_P2(2048, 16, true)
-    TG_P2(3072, 24, true)
-    TG_P2(4096, 16, true)
-    TG_P2(6144, 24, true)
-    TG_P2(8192, 16, true)
-    default: return false;
-  }
+  if constexpr (FMT == FMT_SINGLE && STORE == TG_STORE_FP32) switch (a.fft_n) {  // tg_apply_rweighting
+      TG_P2(256, 8, true)
+      TG_P2(512, 8, true)
+      TG_P2(768, 24, true)
+      TG_P2(1024, 16, true)
+      TG_P2(1536, 24, true)
+      TG_P2(2048, 16, true)
+      TG_P2(3072, 24, true)
+      TG_P2(4096, 16, true)
+      TG_P2(6144, 24, true)
+      TG_P2(8192, 16, true)
+    }
 #undef TG_P2
+  return false;
 }
 
 // threads and shared memory of the generic kernel: two complex ping-pong buffers, and for

@@ -268,7 +268,7 @@ void admit_loop(tg_server *sv) {
     const auto t_adm = std::chrono::steady_clock::now();
     NvtxRange nv("tg.server.admit");
     tg_session *s = nullptr;
-    int rc = session_create_ex(&j->g, &j->o, sv->pool, false, fail_alloc, &s);
+    int rc = session_create_ex(&j->g, &j->o, sv->pool, false, fail_alloc, false, &s);
     if (rc == TG_ERR_OOM && !fail_alloc && j->oom_retries < kMaxOomRetries) {
       // the budget admitted it but the pool could not map the memory yet (frees
       // in flight, fragmentation): give unused memory back, requeue the job at
@@ -557,7 +557,7 @@ int tg_server_submit(tg_server *sv, const tg_job *job, uint64_t *id) {
   j->tag = job->tag;
   // size (and validate) the job with a dry session: no device work
   tg_session *dry = nullptr;
-  int rc = session_create_ex(&j->g, &j->o, nullptr, true, false, &dry);
+  int rc = session_create_ex(&j->g, &j->o, nullptr, true, false, false, &dry);
   if (rc != TG_OK) return rc;
   j->est = dry->dev_bytes;
   session_discard(dry);

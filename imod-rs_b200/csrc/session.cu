@@ -516,16 +516,17 @@ void tg_options_default(tg_options *o) {
 }
 
 int tg_session_create(const tg_geometry *g, const tg_options *opt, tg_session **out) {
-  return tg::session_create_ex(g, opt, nullptr, false, false, out);
+  return tg::session_create_ex(g, opt, nullptr, false, false, false, out);
 }
 
 }  // extern "C"
 
 // pool: allocate stream-ordered from it; dry: compute sizes only (no device
 // work; the returned object holds dev_bytes and must be freed with
-// session_discard); fail_alloc: fault-injection hook (the first allocation fails).
+// session_discard); fail_alloc: fault-injection hook (the first allocation fails);
+// rows_only: the session only R-weights rows (tg_apply_rweighting).
 int tg::session_create_ex(const tg_geometry *g, const tg_options *opt, cudaMemPool_t pool, bool dry,
-                          bool fail_alloc, tg_session **out) {
+                          bool fail_alloc, bool rows_only, tg_session **out) {
   if (!g || !opt || !out) { set_error("null argument"); return TG_ERR_INVALID_ARG; }
   *out = nullptr;
   if (g->nx < 2 || g->ny < 1 || g->nz < 1 || g->nx > 65536 || g->ny > 65535 || g->nz > 4096) {
@@ -678,11 +679,12 @@ int tg::session_create_ex(const tg_geometry *g, const tg_options *opt, cudaMemPo
                   : s->fmt == FMT_OCT   ? (s->ny + 15) / 16 * 2
                                         : s->ny;
 
-  // transform of the register-resident filter kernel, else an FFT plan, else circulant
+  // transform of the register-resident filter kernel, else an FFT plan, else circulant.  A
+  // reconstruction takes only the row's own length: a padded transform is nearer to 64 bits,
+  // but it moves a volume's mean, a small difference of large sums, by up to 1e-2 of itself
+  // and, in half staging, every rounding decision near a midpoint.
   s->fft_n = opt->no_weight || getenv("TG_FILTER_GENERIC") ? 0 : p2_transform_length(s->nx);
-  // half staging rounds the filtered samples, so there another transform of a row (equal to
-  // 1e-6) would move every rounding decision near a midpoint: only the row's own length
-  if (s->store != TG_STORE_FP32 && s->fft_n != s->nx) s->fft_n = 0;
+  if (!rows_only && s->fft_n != s->nx) s->fft_n = 0;
   s->use_conv = !fft_plan(s->nx, &s->plan) && !s->fft_n;
   if (s->nx * 16 > 200 * 1024) { set_error("rows wider than 12800 are not supported"); return fail(TG_ERR_UNSUPPORTED); }
 
@@ -1329,7 +1331,7 @@ int tg_apply_rweighting(float *proj, size_t in_nx, size_t in_ny, size_t nz, floa
   o.device = device;
   o.fill_mode = TG_FILL_ZERO;
   tg_session *s = nullptr;
-  int rc = tg_session_create(&g, &o, &s);
+  int rc = session_create_ex(&g, &o, nullptr, false, false, true, &s);
   if (rc != TG_OK) return rc;
   // SINGLE FP32 staging with no padding holds (row[k], row[k+1]) pairs;
   // element k's first value is the filtered sample.

@@ -82,7 +82,7 @@ struct tg_session {  // one tilt series resident on a device
 namespace tg {
 
 int session_create_ex(const tg_geometry *g, const tg_options *opt, cudaMemPool_t pool, bool dry,
-                      bool fail_alloc, tg_session **out);
+                      bool fail_alloc, bool rows_only, tg_session **out);
 void session_discard(tg_session *s);
 // frees the session's device memory stream-ordered after the work queued on `after`
 void free_session_async(tg_session *s, cudaStream_t after);
