@@ -468,6 +468,7 @@ __device__ __forceinline__ void mma_body(const Job &job, int ntiles, unsigned ch
       // ---------------- producer ----------------
       int b = 0, ph = 1, issued = 0, skipped = -1;
       uint64_t limit = 0;
+      const void *acquired = nullptr;
       for (int t0 = blockIdx.x; t0 < ntiles && !s_abort; t0 += gridDim.x) {
         int t = t0;
         const BpArgs &a = job(t);
@@ -475,7 +476,11 @@ __device__ __forceinline__ void mma_body(const Job &job, int ntiles, unsigned ch
         const Tile q = tile_at(a, t);
         const int nviews = a.nviews, padL = a.padL, skip = a.fault_skip_stage;
         const uint32_t bytes = (uint32_t)(2 * (a.nper / 8) * KW * 16);
-        const void *map = a.tmap;
+        const void *map = job.map(a);
+        if (Job::MAP_IN_MEMORY && map != acquired) {
+          if (lane == 0) tensormap_acquire(map);
+          acquired = map;
+        }
         const int ra = a.rows_alloc;
         int y = q.iy0 / 8;
         limit = a.wait_limit_ns;
@@ -580,11 +585,15 @@ __device__ __forceinline__ void mma_body(const Job &job, int ntiles, unsigned ch
   }
 }
 
-struct OneJob {  // a launch over one series
+struct OneJob {  // a launch over one series, its map a kernel parameter
+  static constexpr bool MAP_IN_MEMORY = false;
   const BpArgs &a;
+  const TensorMap &m;
   __device__ __forceinline__ const BpArgs &operator()(int &) const { return a; }
+  __device__ __forceinline__ const void *map(const BpArgs &) const { return &m; }
 };
 struct ManyJobs {  // tile t belongs to the series j with jobs[j].tile0 <= t < jobs[j+1].tile0
+  static constexpr bool MAP_IN_MEMORY = true;
   const BpArgs *jobs;
   int n;
   __device__ __forceinline__ const BpArgs &operator()(int &t) const {
@@ -597,11 +606,14 @@ struct ManyJobs {  // tile t belongs to the series j with jobs[j].tile0 <= t < j
     t -= __ldg(&jobs[lo].tile0);
     return jobs[lo];
   }
+  __device__ __forceinline__ const void *map(const BpArgs &a) const { return a.tmap; }
 };
 
-template <int KS> __global__ void __launch_bounds__(NTHR, 1) bp_mma_kernel(const __grid_constant__ BpArgs a, int ntiles) {
+template <int KS>
+__global__ void __launch_bounds__(NTHR, 1) bp_mma_kernel(const __grid_constant__ BpArgs a, const __grid_constant__ TensorMap map,
+                                                         int ntiles) {
   extern __shared__ __align__(128) unsigned char sm[];
-  mma_body<KS>(OneJob{a}, ntiles, sm);
+  mma_body<KS>(OneJob{a, map}, ntiles, sm);
 }
 template <int KS>
 __global__ void __launch_bounds__(NTHR, 1) bp_mma_batch_kernel(const BpArgs *__restrict__ jobs, int njobs, int ntiles) {
@@ -619,10 +631,10 @@ template <class K> int set_smem(K kern, int smem) {
   const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   return e == cudaSuccess ? TG_OK : cuda_fail(e, "cudaFuncSetAttribute(bp_mma)");
 }
-template <int KS> int launch_t(const BpArgs &a, int ntiles, cudaStream_t st) {
+template <int KS> int launch_t(const BpArgs &a, const TensorMap &map, int ntiles, cudaStream_t st) {
   const int rc = set_smem(bp_mma_kernel<KS>, Cfg<KS>::SMEM);
   if (rc != TG_OK) return rc;
-  bp_mma_kernel<KS><<<grid_for(ntiles), NTHR, Cfg<KS>::SMEM, st>>>(a, ntiles);
+  bp_mma_kernel<KS><<<grid_for(ntiles), NTHR, Cfg<KS>::SMEM, st>>>(a, map, ntiles);
   return TG_OK;
 }
 template <int KS> int launch_batch_t(const BatchLaunch &bl, cudaStream_t st) {
@@ -664,9 +676,9 @@ long long bp_mma_plan(BpArgs &a) {
 }
 
 // The TMA map of an OCT buffer: boxes of one view's KS*16-element windows of nper/8 blocks in
-// both planes.  Host bytes for BpArgs::tmap (128, copied to the device by the caller).
-int bp_mma_tensor_map(void *pairs, int nviews, int rows_alloc, int PW, int nper, int steps, unsigned char out[128]) {
-  static_assert(sizeof(CUtensorMap) == 128, "tensor map size");
+// both planes.
+int bp_mma_tensor_map(void *pairs, int nviews, int rows_alloc, int PW, int nper, int steps, TensorMap *out) {
+  static_assert(sizeof(CUtensorMap) == sizeof(TensorMap) && alignof(CUtensorMap) <= alignof(TensorMap), "tensor map");
   using Encode = CUresult (*)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *,
                               const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle,
                               CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
@@ -685,7 +697,7 @@ int bp_mma_tensor_map(void *pairs, int nviews, int rows_alloc, int PW, int nper,
                                                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
                                                   CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (e != CUDA_SUCCESS) { set_error("cuTensorMapEncodeTiled failed"); return TG_ERR_CUDA; }
-  memcpy(out, &m, 128);
+  memcpy(out->bytes, &m, sizeof m);
   return TG_OK;
 }
 
@@ -707,12 +719,12 @@ bool bp_mma_pays(int onx, int onz, int ny, int nviews) {
 
 int bp_mma_ntiles(int onx, int onz) { return ((onx - 1 + 7) / HX + 1) * ((onz - 1 + 4) / HZ + 1); }
 
-int launch_bp_mma(const BpArgs &a0, int steps, cudaStream_t st, int *ntiles) {
+int launch_bp_mma(const BpArgs &a0, const TensorMap &map, int steps, cudaStream_t st, int *ntiles) {
   BpArgs a = a0;
   const long long n = bp_mma_plan(a);
   if (n >= (1ll << 31) - (1ll << 20)) { set_error("too many tiles"); return TG_ERR_UNSUPPORTED; }
   if (ntiles) *ntiles = a.ntiles_xz;
-  return steps == 1 ? launch_t<1>(a, (int)n, st) : launch_t<2>(a, (int)n, st);
+  return steps == 1 ? launch_t<1>(a, map, (int)n, st) : launch_t<2>(a, map, (int)n, st);
 }
 
 int launch_bp_mma_batch(const BatchLaunch &bl, int steps, cudaStream_t st) {

@@ -39,13 +39,18 @@ __device__ __forceinline__ void bulk_g2s(uint32_t dst, const void *src, uint32_t
       "l"(src), "r"(bytes), "r"(bar)
       : "memory");
 }
-// TMA box of a 3-D tensor map (in global memory): x counts elements of the innermost
-// dimension, its byte offset a multiple of 16
+// TMA box of a 3-D tensor map: x counts elements of the innermost dimension, its byte offset
+// a multiple of 16.  The map is a kernel parameter, or in global memory and acquired first.
 __device__ __forceinline__ void tma_box3(uint32_t dst, const void *map, int x, int y, int z, uint32_t bar) {
   asm volatile(
       "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(dst),
       "l"(map), "r"(x), "r"(y), "r"(z), "r"(bar)
       : "memory");
+}
+// Before a CTA's first use of a tensor map that the host copied to global memory: copies read
+// their map through a cache of its own, which may still hold what was at this address before.
+__device__ __forceinline__ void tensormap_acquire(const void *map) {
+  asm volatile("fence.proxy.tensormap::generic.acquire.sys [%0], 128;" ::"l"(map) : "memory");
 }
 __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");

@@ -327,7 +327,7 @@ FilterArgs filter_args(tg_session *s, bool residual) {
 int launch_bp(tg_session *s, int mode, int *ntiles) {
   BpArgs a = bp_args(s, mode);
   auto rows = [&](const BpArgs &b, int *nt) {
-    if (s->mma_steps) return launch_bp_mma(b, s->mma_steps, s->st, nt);
+    if (s->mma_steps) return launch_bp_mma(b, s->tmap, s->mma_steps, s->st, nt);
     return launch_bp_fast(b, s->store, fast_zf(s), s->variant < 0 ? 0 : s->variant, s->st, nt);
   };
   if (s->fast) return rows(a, ntiles);
@@ -809,12 +809,11 @@ int tg::session_create_ex(const tg_geometry *g, const tg_options *opt, cudaMemPo
       (ce = cudaMemcpyAsync(s->d_vg2, vg2.data(), vg2.size() * 16, cudaMemcpyHostToDevice, s->st)) ||
       (ce = cudaMemcpyAsync(s->d_stretch, stretch.data(), stretch.size() * 4, cudaMemcpyHostToDevice, s->st)))
     return fail(cuda_fail(ce, "cudaMemcpy(setup)"));
-  unsigned char tmap[128];
   if (s->mma_steps) {
     BpArgs a = bp_args(s, 0);
     bp_mma_plan(a);
-    if ((rc = bp_mma_tensor_map(s->d_pairs, s->nviews, s->rows_alloc, s->PW, a.nper, s->mma_steps, tmap)) != TG_OK) return fail(rc);
-    if ((ce = cudaMemcpyAsync(s->d_tmap, tmap, 128, cudaMemcpyHostToDevice, s->st))) return fail(cuda_fail(ce, "cudaMemcpy(setup)"));
+    if ((rc = bp_mma_tensor_map(s->d_pairs, s->nviews, s->rows_alloc, s->PW, a.nper, s->mma_steps, &s->tmap)) != TG_OK) return fail(rc);
+    if ((ce = cudaMemcpyAsync(s->d_tmap, &s->tmap, sizeof s->tmap, cudaMemcpyHostToDevice, s->st))) return fail(cuda_fail(ce, "cudaMemcpy(setup)"));
   }
   if (!any_stretch) {
     if (pool) cudaFreeAsync(s->d_stretch, s->st);

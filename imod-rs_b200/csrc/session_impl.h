@@ -20,7 +20,8 @@ struct tg_session {  // one tilt series resident on a device
   // views into xtb, then launch_xt_blend blends two rows per voxel into the volume
   bool xt_split = false;
   int mma_steps = 0;       // fast or row-sum path on the tensor-core back-projector: its K steps (else 0)
-  void *d_tmap = nullptr;  // TMA map of d_pairs on that path
+  tg::TensorMap tmap{};    // TMA map of d_pairs on that path, and its copy for batched launches
+  void *d_tmap = nullptr;
   float oct_gain = 1.0f;   // oct_scale's gain on that path
   float *xtb = nullptr;    // row sums (d_xtb, or the reprojector's FP32 copy, which is dead then)
   float *d_xtb = nullptr;

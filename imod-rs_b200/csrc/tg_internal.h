@@ -158,7 +158,7 @@ struct BpArgs {
   int nper;
   const int *nonfinite;
   const unsigned *range;
-  const void *tmap;         // TMA map of pairs (bp_mma_tensor_map), in device memory
+  const void *tmap;         // batched launches: the series' TensorMap, in device memory
   float gain;
   int pad_;
 };
@@ -188,8 +188,9 @@ int bp_mma_steps(const std::vector<float4> &vg);
 long long bp_mma_plan(BpArgs &a);  // fills the tile grid (nbx, ntiles_xz, nper); returns the tiles
 int bp_mma_ntiles(int onx, int onz);
 bool bp_mma_pays(int onx, int onz, int ny, int nviews);
-int bp_mma_tensor_map(void *pairs, int nviews, int rows_alloc, int PW, int nper, int steps, unsigned char out[128]);
-int launch_bp_mma(const BpArgs &a, int steps, cudaStream_t st, int *ntiles_out);
+struct alignas(64) TensorMap { unsigned char bytes[128]; };  // a CUtensorMap
+int bp_mma_tensor_map(void *pairs, int nviews, int rows_alloc, int PW, int nper, int steps, TensorMap *out);
+int launch_bp_mma(const BpArgs &a, const TensorMap &map, int steps, cudaStream_t st, int *ntiles_out);
 int launch_bp_mma_batch(const BatchLaunch &bl, int steps, cudaStream_t st);
 // General kernel: x-tilt, z-factor, local alignment, SINGLE format.
 int launch_bp_general(const BpArgs &a, int store, cudaStream_t st, int *ntiles_out);
