@@ -180,7 +180,23 @@ __device__ __noinline__ void sum_views(const BpArgs &a, float dx, float dz, int 
 
 template <int N> __device__ __forceinline__ void reg_inc() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
 template <int N> __device__ __forceinline__ void reg_dec() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
-__device__ __forceinline__ void cons_sync() { asm volatile("bar.sync 1, %0;" ::"n"(NCONS * 32) : "memory"); }
+// Barrier of all consumer threads, and whether q held in any of them: every thread gets the
+// same answer, whatever another role writes to the abort flag meanwhile.
+__device__ __forceinline__ bool cons_any(bool q) {
+  uint32_t r;
+  __syncwarp();
+  asm volatile(
+      "{\n .reg .pred p, q;\n setp.ne.u32 q, %1, 0;\n bar.red.or.pred p, 1, %2, q;\n selp.u32 %0, 1, 0, p;\n}\n"
+      : "=r"(r)
+      : "r"((uint32_t)q), "n"(NCONS * 32)
+      : "memory");
+  return r != 0;
+}
+// A wait of a whole warp: its lanes agree on the outcome, so that none leaves the loop
+// while others go on to the warp-wide instructions behind the wait.
+__device__ __forceinline__ bool warp_poll(uint32_t bar, uint32_t parity, volatile int *abort, uint64_t limit) {
+  return __all_sync(0xffffffffu, poll_phase(bar, parity, abort, limit));
+}
 
 // A wait gave up: the series of this CTA's unfinished tiles report it.
 template <class Job> __device__ __noinline__ void abandon(const Job &job, int t0, int ntiles) {
@@ -231,10 +247,6 @@ __device__ __forceinline__ void mma_body(const Job &job, int ntiles, unsigned ch
     StatPartial *part = reinterpret_cast<StatPartial *>(sm + NST * C::STAGE + C::TR);
     int ph = 0;  // bit e: phase of tensor-memory buffer e
     for (int t0 = blockIdx.x; t0 < ntiles; t0 += gridDim.x) {
-      if (s_abort) {
-        if (lane == 0) abandon(job, t0, ntiles);
-        break;
-      }
       int t = t0;
       const BpArgs &a = job(t);
       const Tile q = tile_at(a, t);
@@ -246,16 +258,12 @@ __device__ __forceinline__ void mma_body(const Job &job, int ntiles, unsigned ch
       float acc[128];
 #pragma unroll
       for (int i = 0; i < 128; ++i) acc[i] = 0.0f;
+      bool go = true;
       if (*a.nonfinite == 0) {
         const uint64_t limit = a.wait_limit_ns;
-        bool go = true;
         for (int i = 0; 2 * i < nviews; ++i) {
           const int e = i & 1;
-          if (!poll_phase(smem_u32(&tfull[e]), (ph >> e) & 1, &s_abort, limit)) {
-            go = false;
-            break;
-          }
-          __syncwarp();
+          if (!(go = warp_poll(smem_u32(&tfull[e]), (ph >> e) & 1, &s_abort, limit))) break;
           tcgen05_after_sync();
           const uint32_t src = tm + ((uint32_t)(warp & 3) << 21) + e * 256 + c0;
 #pragma unroll
@@ -273,11 +281,7 @@ __device__ __forceinline__ void mma_body(const Job &job, int ntiles, unsigned ch
           if (cnt == 0 && lane == 0) mbar_arrive(smem_u32(&tempty[e]));
           ph ^= 1 << e;
         }
-        if (!go) {
-          s_abort = 1;
-          if (lane == 0) abandon(job, t0, ntiles);
-          break;
-        }
+        if (!go) s_abort = 1;
       } else {
         const float dx = __fsub_rn((float)min(max(ox, 0), onx - 1), a.ocx), dz = __fsub_rn((float)min(max(oz, 0), onz - 1), a.cz);
 #pragma unroll 1
@@ -288,6 +292,13 @@ __device__ __forceinline__ void mma_body(const Job &job, int ntiles, unsigned ch
           for (int i = 0; i < 128; ++i)
             if (i / 8 == b) acc[i] = s8[i % 8];
         }
+      }
+      // all consumer warps store this tile, or none does: the barriers of the epilogue expect
+      // them all.  (Behind this one, the previous tile's statistics have been read.)
+      if (cons_any(!go || s_abort)) {
+        s_abort = 1;
+        if (lane == 0) abandon(job, t0, ntiles);
+        break;
       }
       // ---------------- epilogue ----------------
       const size_t sl = (size_t)onz * onx;
@@ -360,7 +371,7 @@ __device__ __forceinline__ void mma_body(const Job &job, int ntiles, unsigned ch
           }
           __syncwarp();
         }
-        cons_sync();
+        cons_any(false);
         if (tid < q.n && q.iy0 + tid < a.ny) {
           StatPartial p = part[tid * 4];
 #pragma unroll
@@ -372,7 +383,6 @@ __device__ __forceinline__ void mma_body(const Job &job, int ntiles, unsigned ch
           }
           a.partial[(size_t)(q.iy0 + tid) * a.ntiles_xz + q.idx] = p;
         }
-        cons_sync();
       }
     }
   } else if (warp < NCONS + NWGT) {
@@ -381,7 +391,7 @@ __device__ __forceinline__ void mma_body(const Job &job, int ntiles, unsigned ch
     const int row = tid - NCONS * 32;
     const int2 vox = hex_voxel(min(row, NVOX - 1));
     int b = 0, ph = 1;
-    for (int t0 = blockIdx.x; t0 < ntiles && !s_abort; t0 += gridDim.x) {
+    for (int t0 = blockIdx.x; t0 < ntiles && !__any_sync(0xffffffffu, s_abort); t0 += gridDim.x) {
       int t = t0;
       const BpArgs &a = job(t);
       if (*a.nonfinite) continue;
@@ -440,19 +450,13 @@ __device__ __forceinline__ void mma_body(const Job &job, int ntiles, unsigned ch
         g0 = __ldg(vg + min(v + 2, nviews - 1));
         g1 = __ldg(vg + min(v + 3, nviews - 1));
         const bool two = v + 1 < nviews;
-        if (!poll_phase(smem_u32(&empty[b]), ph, &s_abort, limit)) {
-          go = false;
-          break;
-        }
+        if (!(go = warp_poll(smem_u32(&empty[b]), ph, &s_abort, limit))) break;
         const uint32_t dst = ring + b * C::STAGE + row * 16;
         store_row(wa, dst);
         if (two) store_row(wb, dst + C::VIEW);
         fence_proxy_async();
         // the first weight warp also waits for the windows, so that the issuing threads wait once
-        if (warp == NCONS && !poll_phase(smem_u32(&fullb[b]), ph ^ 1, &s_abort, limit)) {
-          go = false;
-          break;
-        }
+        if (warp == NCONS && !(go = warp_poll(smem_u32(&fullb[b]), ph ^ 1, &s_abort, limit))) break;
         __syncwarp();
         if (lane == 0) mbar_arrive(smem_u32(&full[b]));
         if (++b == NST) { b = 0; ph ^= 1; }
@@ -469,7 +473,7 @@ __device__ __forceinline__ void mma_body(const Job &job, int ntiles, unsigned ch
       int b = 0, ph = 1, issued = 0, skipped = -1;
       uint64_t limit = 0;
       const void *acquired = nullptr;
-      for (int t0 = blockIdx.x; t0 < ntiles && !s_abort; t0 += gridDim.x) {
+      for (int t0 = blockIdx.x; t0 < ntiles && !__any_sync(0xffffffffu, s_abort); t0 += gridDim.x) {
         int t = t0;
         const BpArgs &a = job(t);
         if (*a.nonfinite) continue;
@@ -490,9 +494,7 @@ __device__ __forceinline__ void mma_body(const Job &job, int ntiles, unsigned ch
           if ((v & 31) == 0) k0s = window_start<KW>(a, q, v + lane);
           const int ka = __shfl_sync(0xffffffffu, k0s, v & 31), kb = __shfl_sync(0xffffffffu, k0s, (v + 1) & 31);
           const bool two = v + 1 < nviews;
-          go = poll_phase(smem_u32(&empty[b]), ph, &s_abort, limit);
-          go = __all_sync(0xffffffffu, go && !s_abort);  // one decision for the warp
-          if (!go) break;
+          if (!(go = warp_poll(smem_u32(&empty[b]), ph, &s_abort, limit))) break;
           if (v / 2 == skip) {  // test hook: no copy, fullb[b] never completes
             skipped = issued++;
           } else {
@@ -512,7 +514,7 @@ __device__ __forceinline__ void mma_body(const Job &job, int ntiles, unsigned ch
           break;
         }
       }
-      if (s_abort && lane == 0)  // no copy may land after the CTA exits
+      if (lane == 0)  // no copy may land after the CTA exits (another role may give up any time)
         for (int g = max(0, issued - NST); g < issued; ++g)
           if (g != skipped) poll_phase(smem_u32(&fullb[g % NST]), (g / NST) & 1, nullptr, limit);
     } else if (warp <= 14 && lane == 0) {

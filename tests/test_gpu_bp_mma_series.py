@@ -62,3 +62,55 @@ def test_series_that_follow_each_other_on_the_same_memory(how, monkeypatch):
             assert rel_l2(v, want[i]) <= TOL, (turn, i)
     if sv:
         sv.close()
+
+
+# ---- a wait that runs out: a status, no endless barrier, and the session works again ----
+
+def fails(call):
+    with pytest.raises(T.TiltGpuError) as e:
+        call()
+    assert e.value.code == -4 and "timed out" in str(e.value)
+
+
+@pytest.mark.parametrize("sirt", [0, 2])
+@pytest.mark.parametrize("nz,skip", [(31, 1), (31, 15), (31, 0), (6, 2), (3, 1), (1, 0)])
+@pytest.mark.parametrize("ny", [40, 272])  # consumer warps with and without columns of their own
+def test_bounded_wait_times_out_and_session_recovers(nz, skip, sirt, ny):
+    ang = np.linspace(-60, 60, nz).astype(np.float32)
+    kw = dict(thickness=61, sirt=sirt, sirt_relax=0.5) if sirt else dict(thickness=61)
+    with session(200, ny, ang, smooth_stack(nz, ny, 200, seed=nz), **kw) as s:
+        assert s.kernel_info()["variant_name"] == "tcgen05-hex126"
+        s.reconstruct()
+        good, st = s.download()
+        s.inject_wait_fault(skip_stage=skip, wait_limit_us=5000)
+        fails(s.reconstruct)
+        s.inject_wait_fault(-1, 0)
+        s.reconstruct()
+        again, st2 = s.download()
+    np.testing.assert_array_equal(again, good)
+    assert st == st2
+
+
+def test_bounded_wait_in_a_batch():
+    ang = [np.linspace(-55, 55, nz).astype(np.float32) for _, _, nz, _ in SHAPES]
+    ss = [session(nx, ny, ang[i], smooth_stack(nz, ny, nx, seed=20 + i), thickness=th, sirt=2 * (i % 2), sirt_relax=0.5)
+          for i, (nx, ny, nz, th) in enumerate(SHAPES)]
+    b = T.Batch()
+    for s in ss:
+        b.add(s)
+    b.reconstruct()
+    good = [s.download()[0] for s in ss]
+    ss[2].inject_wait_fault(skip_stage=3, wait_limit_us=5000)
+    fails(b.reconstruct)
+    for s in ss:  # series whose tiles were in the same blocks report it too
+        try:
+            s.synchronize()
+        except T.TiltGpuError as e:
+            assert e.code == -4
+    ss[2].inject_wait_fault(-1, 0)
+    b.reconstruct()
+    for s, g in zip(ss, good):
+        np.testing.assert_array_equal(s.download()[0], g)
+    b.close()
+    for s in ss:
+        s.close()
