@@ -95,18 +95,6 @@ __device__ __forceinline__ bool poll_phase(uint32_t bar, uint32_t parity, volati
   return wait_phase(bar, parity, abort, limit_ns);
 }
 
-// poll_phase on two barriers: a wait's result takes some 170 cycles to arrive even when
-// the phase has completed, so both are asked for at once
-__device__ __forceinline__ bool wait_phases(uint32_t bar0, uint32_t parity0, uint32_t bar1, uint32_t parity1,
-                                            volatile int *abort, uint64_t limit_ns) {
-#pragma unroll 1
-  for (int i = 0; i < 64; ++i) {
-    const bool x = mbar_try_wait(bar0, parity0), y = mbar_try_wait(bar1, parity1);
-    if (x & y) return true;
-  }
-  return wait_phase(bar0, parity0, abort, limit_ns) && wait_phase(bar1, parity1, abort, limit_ns);
-}
-
 constexpr float MAGIC = 12582912.0f;      // 1.5 * 2^23
 constexpr uint32_t MAGIC_BITS = 0x4B400000u;
 
