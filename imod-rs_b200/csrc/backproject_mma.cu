@@ -33,7 +33,8 @@
 //               and plane instead: 62 cycles each, 64 a view, measured 4x slower.)
 //   warps 13-14 one thread each issues the tcgen05.mma's of every other view into its
 //               tensor-memory buffer of 256 columns and commits
-// A tile's epilogue overlaps the next tile's first views.
+// A tile's epilogue overlaps the next tile's first views.  Blocks of slices with values
+// that are not finite take bp_oct_kernel, launched behind it.
 #include <cuda.h>
 #include <cuda_fp16.h>
 
@@ -151,16 +152,16 @@ __device__ __forceinline__ void accumulate(float (&acc)[128], int c, const float
   }
 }
 
-// The samples of a voxel in 8 slices summed over the views without the tensor cores,
-// for series with an infinite or NaN staged value: a product with the zeros of W would
-// spread it to voxels that do not sample it.
-__device__ __noinline__ void sum_views(const BpArgs &a, float dx, float dz, int blk, float *s8) {
+// The samples of a voxel in 8 slices summed over the views without the tensor cores
+__device__ __forceinline__ void sum_views(const BpArgs &a, float dx, float dz, int blk, float (&s8)[8]) {
+#pragma unroll
   for (int j = 0; j < 8; ++j) s8[j] = 0.0f;
   const size_t plane = (size_t)a.nviews * a.rows_alloc * a.PW;
   auto value = [](uint32_t hi, uint32_t lo, int i) {
     const float h = half_val(hi, i);
     return fabsf(h) <= 65504.0f ? h + half_val(lo, i) : h;
   };
+#pragma unroll 2
   for (int v = 0; v < a.nviews; ++v) {
     const float x = position(dx, dz, __ldg(&a.vg[v]), a.cx);
     const float tt = __fadd_rd(x, MAGIC);
@@ -171,6 +172,7 @@ __device__ __noinline__ void sum_views(const BpArgs &a, float dx, float dz, int 
     const uint4 *e = reinterpret_cast<const uint4 *>(a.pairs) + ((size_t)v * a.rows_alloc + blk) * a.PW + (k + a.padL);
     const uint4 u0 = __ldg(e), z0 = __ldg(e + plane), u1 = in ? __ldg(e + 1) : u0, z1 = in ? __ldg(e + 1 + plane) : z0;
     const uint32_t *p0 = &u0.x, *q0 = &z0.x, *p1 = &u1.x, *q1 = &z1.x;
+#pragma unroll
     for (int j = 0; j < 8; ++j) {
       const float v0 = value(p0[j / 2], q0[j / 2], j & 1);
       s8[j] += in ? v0 * (1.0f - f) + value(p1[j / 2], q1[j / 2], j & 1) * f : v0;
@@ -259,40 +261,28 @@ __device__ __forceinline__ void mma_body(const Job &job, int ntiles, unsigned ch
 #pragma unroll
       for (int i = 0; i < 128; ++i) acc[i] = 0.0f;
       bool go = true;
-      if (*a.nonfinite == 0) {
-        const uint64_t limit = a.wait_limit_ns;
-        for (int i = 0; 2 * i < nviews; ++i) {
-          const int e = i & 1;
-          if (!(go = warp_poll(smem_u32(&tfull[e]), (ph >> e) & 1, &s_abort, limit))) break;
-          tcgen05_after_sync();
-          const uint32_t src = tm + ((uint32_t)(warp & 3) << 21) + e * 256 + c0;
+      const uint64_t limit = a.wait_limit_ns;
+      for (int i = 0; 2 * i < nviews; ++i) {
+        const int e = i & 1;
+        if (!(go = warp_poll(smem_u32(&tfull[e]), (ph >> e) & 1, &s_abort, limit))) break;
+        tcgen05_after_sync();
+        const uint32_t src = tm + ((uint32_t)(warp & 3) << 21) + e * 256 + c0;
 #pragma unroll
-          for (int c = 0; c < 4; ++c)
-            if (32 * c < cnt) {
-              float r[32];
-              tmem_ld32(src + 32 * c, r);
-              if (32 * (c + 1) >= cnt) {  // all read: the buffer is free
-                tcgen05_before_sync();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(smem_u32(&tempty[e]));
-              }
-              accumulate(acc, c, r);
+        for (int c = 0; c < 4; ++c)
+          if (32 * c < cnt) {
+            float r[32];
+            tmem_ld32(src + 32 * c, r);
+            if (32 * (c + 1) >= cnt) {  // all read: the buffer is free
+              tcgen05_before_sync();
+              __syncwarp();
+              if (lane == 0) mbar_arrive(smem_u32(&tempty[e]));
             }
-          if (cnt == 0 && lane == 0) mbar_arrive(smem_u32(&tempty[e]));
-          ph ^= 1 << e;
-        }
-        if (!go) s_abort = 1;
-      } else {
-        const float dx = __fsub_rn((float)min(max(ox, 0), onx - 1), a.ocx), dz = __fsub_rn((float)min(max(oz, 0), onz - 1), a.cz);
-#pragma unroll 1
-        for (int b = 0; b < cnt / 8; ++b) {
-          float s8[8];
-          sum_views(a, dx, dz, (q.iy0 + c0) / 8 + b, s8);
-#pragma unroll
-          for (int i = 0; i < 128; ++i)
-            if (i / 8 == b) acc[i] = s8[i % 8];
-        }
+            accumulate(acc, c, r);
+          }
+        if (cnt == 0 && lane == 0) mbar_arrive(smem_u32(&tempty[e]));
+        ph ^= 1 << e;
       }
+      if (!go) s_abort = 1;
       // all consumer warps store this tile, or none does: the barriers of the epilogue expect
       // them all.  (Behind this one, the previous tile's statistics have been read.)
       if (cons_any(!go || s_abort)) {
@@ -309,6 +299,8 @@ __device__ __forceinline__ void mma_body(const Job &job, int ntiles, unsigned ch
         for (int i = 0; i < 128; ++i) acc[i] = __fmul_rn(acc[i], inv);
       }
       const int iy = q.iy0 + c0, ny = min(cnt, a.ny - iy);  // slices of this warp inside the volume
+      // its blocks of 8 slices that hold a value that is not finite: bp_oct_kernel stores those
+      const unsigned skip = __ballot_sync(0xffffffffu, 8 * lane < ny && __ldg(a.flags + min(iy / 8 + lane, (a.ny - 1) / 8)));
       float *out = a.vol + ((size_t)iy * onz + oz) * onx + ox;
       const int mode = a.mode;
       if (mode == 2) {  // SIRT update vol += relax * v: 8 old values loaded together before their stores
@@ -316,19 +308,20 @@ __device__ __forceinline__ void mma_body(const Job &job, int ntiles, unsigned ch
 #pragma unroll
         for (int j0 = 0; j0 < 128; j0 += 8) {
           if (j0 >= ny) break;
+          const bool put = ok && !((skip >> (j0 / 8)) & 1);
           float old[8];
 #pragma unroll
-          for (int j = 0; j < 8; ++j) old[j] = (ok && j0 + j < ny) ? out[(size_t)j * sl] : 0.0f;
+          for (int j = 0; j < 8; ++j) old[j] = (put && j0 + j < ny) ? out[(size_t)j * sl] : 0.0f;
 #pragma unroll
           for (int j = 0; j < 8; ++j)
-            if (ok && j0 + j < ny)
+            if (put && j0 + j < ny)
               out[(size_t)j * sl] = __fadd_rn(old[j], __fmul_rn(relax, __fmul_rn(acc[j0 + j], inv_n)));
           out += 8 * sl;
         }
       } else if (mode == 1) {
 #pragma unroll
         for (int j = 0; j < 128; ++j) {
-          if (ok && j < ny) *out = __fmul_rn(acc[j], inv_n);
+          if (ok && j < ny && !((skip >> (j / 8)) & 1)) *out = __fmul_rn(acc[j], inv_n);
           out += sl;
         }
       } else {
@@ -340,7 +333,7 @@ __device__ __forceinline__ void mma_body(const Job &job, int ntiles, unsigned ch
 #pragma unroll
           for (int j = 0; j < 16; ++j) {
             const float y = __fadd_rn(__fmul_rn(__fmul_rn(__fmul_rn(acc[j0 + j], inv_n), dw), os), oa);
-            if (ok && j0 + j < ny) *out = y;
+            if (ok && j0 + j < ny && !((skip >> ((j0 + j) / 8)) & 1)) *out = y;
             out += sl;
             tr[j * 33 + lane] = y;
           }
@@ -372,7 +365,7 @@ __device__ __forceinline__ void mma_body(const Job &job, int ntiles, unsigned ch
           __syncwarp();
         }
         cons_any(false);
-        if (tid < q.n && q.iy0 + tid < a.ny) {
+        if (tid < q.n && q.iy0 + tid < a.ny && !__ldg(a.flags + (q.iy0 + tid) / 8)) {
           StatPartial p = part[tid * 4];
 #pragma unroll
           for (int w = 1; w < 4; ++w) {
@@ -394,7 +387,6 @@ __device__ __forceinline__ void mma_body(const Job &job, int ntiles, unsigned ch
     for (int t0 = blockIdx.x; t0 < ntiles && !__any_sync(0xffffffffu, s_abort); t0 += gridDim.x) {
       int t = t0;
       const BpArgs &a = job(t);
-      if (*a.nonfinite) continue;
       const Tile q = tile_at(a, t);
       const int nviews = a.nviews, nx2 = a.nx - 2;
       const int ox = q.ox + vox.x, oz = q.oz + vox.y;
@@ -476,7 +468,6 @@ __device__ __forceinline__ void mma_body(const Job &job, int ntiles, unsigned ch
       for (int t0 = blockIdx.x; t0 < ntiles && !__any_sync(0xffffffffu, s_abort); t0 += gridDim.x) {
         int t = t0;
         const BpArgs &a = job(t);
-        if (*a.nonfinite) continue;
         const Tile q = tile_at(a, t);
         const int nviews = a.nviews, padL = a.padL, skip = a.fault_skip_stage;
         const uint32_t bytes = (uint32_t)(2 * (a.nper / 8) * KW * 16);
@@ -531,7 +522,6 @@ __device__ __forceinline__ void mma_body(const Job &job, int ntiles, unsigned ch
       for (int t0 = blockIdx.x; t0 < ntiles && go && !s_abort; t0 += gridDim.x) {
         int t = t0;
         const BpArgs &a = job(t);
-        if (*a.nonfinite) continue;
         const Tile q = tile_at(a, t);
         const int nviews = a.nviews, npairs = (nviews + 1) / 2;
         limit = a.wait_limit_ns;
@@ -623,12 +613,88 @@ __global__ void __launch_bounds__(NTHR, 1) bp_mma_batch_kernel(const BpArgs *__r
   mma_body<KS>(ManyJobs{jobs, njobs}, ntiles, sm);
 }
 
-int grid_for(int ntiles) {
+// The blocks of 8 slices that hold a value that is not finite, which a product with the zeros of
+// W spreads to the voxels of its slice that do not sample it: the same tiles, one voxel
+// per thread, sample by sample.  A kernel of its own, so that the tensor-core kernel's warps
+// never wait for such a tile and the rest of a series keeps its speed; with no such block a
+// CTA reads one word and ends.
+constexpr int OCT_T = 128;
+__device__ __forceinline__ void oct_blocks(const BpArgs &a, int ntiles_xz) {
+  const int nblk = (a.ny + 7) / 8;
+  if (!a.flags[nblk]) return;
+  __shared__ StatPartial part[OCT_T / 32][8];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int2 vox = hex_voxel(min(tid, NVOX - 1));
+  const float inv = oct_scale(a.range, a.gain, true);
+  int first = blockIdx.x;  // this CTA's first tile of the next flagged block
+  for (int b0 = 0; b0 < nblk; b0 += 32) {
+    unsigned todo = __ballot_sync(0xffffffffu, b0 + lane < nblk && a.flags[min(b0 + lane, nblk - 1)]);
+    for (; todo; todo &= todo - 1) {
+      const int blk = b0 + __ffs(todo) - 1, iy = 8 * blk;
+      int t = first;
+      for (; t < ntiles_xz; t += gridDim.x) {
+        const Tile q = tile_at(a, t);
+        const int ox = q.ox + vox.x, oz = q.oz + vox.y;
+        const bool ok = tid < NVOX && ox >= 0 && ox < a.onx && oz >= 0 && oz < a.onz;
+        const float dx = __fsub_rn((float)min(max(ox, 0), a.onx - 1), a.ocx);
+        const float dz = __fsub_rn((float)min(max(oz, 0), a.onz - 1), a.cz);
+        float s8[8];
+        sum_views(a, dx, dz, blk, s8);
+        float *out = a.vol + ((size_t)iy * a.onz + oz) * a.onx + ox;
+        const size_t sl = (size_t)a.onz * a.onx;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          const bool put = ok && iy + j < a.ny;
+          float y = __fmul_rn(__fmul_rn(s8[j], inv), a.inv_n);
+          if (a.mode == 2 && put) y = __fadd_rn(out[j * sl], __fmul_rn(a.relax, y));
+          if (a.mode == 0) {
+            y = __fadd_rn(__fmul_rn(__fmul_rn(y, a.dw), a.os), a.oa);
+            float mn = put ? fminf(3.40282347e+38f, y) : 3.40282347e+38f, mx = put ? fmaxf(-3.40282347e+38f, y) : -3.40282347e+38f;
+            double sum = put ? (double)y : 0.0;
+            for (int o = 16; o > 0; o >>= 1) {
+              mn = fminf(mn, __shfl_xor_sync(0xffffffffu, mn, o));
+              mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+              sum += __shfl_xor_sync(0xffffffffu, sum, o);
+            }
+            if (lane == 0) {
+              part[warp][j].mn = mn;
+              part[warp][j].mx = mx;
+              part[warp][j].sum = sum;
+            }
+          }
+          if (put) out[j * sl] = y;
+        }
+        if (a.mode == 0) {
+          __syncthreads();
+          if (tid < 8 && iy + tid < a.ny) {
+            StatPartial p = part[0][tid];
+            for (int w = 1; w < OCT_T / 32; ++w) {
+              p.mn = fminf(p.mn, part[w][tid].mn);
+              p.mx = fmaxf(p.mx, part[w][tid].mx);
+              p.sum += part[w][tid].sum;
+            }
+            a.partial[(size_t)(iy + tid) * ntiles_xz + q.idx] = p;
+          }
+          __syncthreads();
+        }
+      }
+      first = t - ntiles_xz;  // blocks follow each other in one tile sequence over the CTAs
+    }
+  }
+}
+__global__ void __launch_bounds__(OCT_T) bp_oct_kernel(const __grid_constant__ BpArgs a) { oct_blocks(a, a.ntiles_xz); }
+__global__ void __launch_bounds__(OCT_T) bp_oct_batch_kernel(const BpArgs *__restrict__ jobs, int njobs) {
+  for (int j = 0; j < njobs; ++j) oct_blocks(jobs[j], jobs[j].ntiles_xz);
+}
+
+int sm_count() {
   int dev = 0, nsm = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-  return std::max(1, std::min(ntiles, nsm));
+  return nsm;
 }
+int grid_for(int ntiles) { return std::max(1, std::min(ntiles, sm_count())); }
+int oct_grid(int ntiles) { return std::max(1, std::min(ntiles, 8 * sm_count())); }
 template <class K> int set_smem(K kern, int smem) {
   const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   return e == cudaSuccess ? TG_OK : cuda_fail(e, "cudaFuncSetAttribute(bp_mma)");
@@ -637,12 +703,14 @@ template <int KS> int launch_t(const BpArgs &a, const TensorMap &map, int ntiles
   const int rc = set_smem(bp_mma_kernel<KS>, Cfg<KS>::SMEM);
   if (rc != TG_OK) return rc;
   bp_mma_kernel<KS><<<grid_for(ntiles), NTHR, Cfg<KS>::SMEM, st>>>(a, map, ntiles);
+  bp_oct_kernel<<<oct_grid(ntiles), OCT_T, 0, st>>>(a);
   return TG_OK;
 }
 template <int KS> int launch_batch_t(const BatchLaunch &bl, cudaStream_t st) {
   const int rc = set_smem(bp_mma_batch_kernel<KS>, Cfg<KS>::SMEM);
   if (rc != TG_OK) return rc;
   bp_mma_batch_kernel<KS><<<grid_for(bl.ntiles), NTHR, Cfg<KS>::SMEM, st>>>(bl.jobs, bl.njobs, bl.ntiles);
+  bp_oct_batch_kernel<<<oct_grid(bl.ntiles), OCT_T, 0, st>>>(bl.jobs, bl.njobs);
   return TG_OK;
 }
 

@@ -81,7 +81,7 @@ int batch_bp(tg_batch *b, const std::vector<tg_session *> &ss, const std::vector
     int rc = launch_bp_group(kv.first, bl, b->st);
     if (rc != TG_OK) return rc;
     TG_CUDA(cudaGetLastError());
-    ++*launches;
+    *launches += bp_group_launches(kv.first);
     ++b->persistent_launches;
   }
   return TG_OK;

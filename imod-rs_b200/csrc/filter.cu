@@ -302,7 +302,7 @@ template <int STORE> __device__ __forceinline__ void range_report(const FilterAr
 
 // OCT staging, rows 2j and 2j+1 of element e: two of the element's eight halves in each
 // plane.  Infinities and NaN are noted in `top` (the largest magnitude bits of any
-// half): the tensor-core back-projector then takes its element-by-element form.
+// half): the tensor-core back-projector then leaves this block of rows to bp_oct_kernel.
 struct OctWriter {
   uint32_t *out;     // this row pair's word of element 0 (elements are 4 words apart)
   size_t plane;      // words to the second plane
@@ -320,8 +320,8 @@ struct OctWriter {
     out[(size_t)e * 4] = w;
     out[(size_t)e * 4 + plane] = Pack<TG_STORE_FP16>::h2(__fsub_rn(x0, __low2float(h)), __fsub_rn(x1, __high2float(h)));
   }
-  __device__ __forceinline__ void report(const FilterArgs &a) const {
-    if ((top & 0xffffu) >= 0x7c00u || (top >> 16) >= 0x7c00u) *a.nonfinite = 1;
+  __device__ __forceinline__ void report(const FilterArgs &a, int jp) const {
+    if ((top & 0xffffu) >= 0x7c00u || (top >> 16) >= 0x7c00u) a.flags[jp >> 2] = a.flags[(a.ny + 7) / 8] = 1;
   }
 };
 
@@ -499,7 +499,7 @@ __global__ void __launch_bounds__(256) filter_kernel(FilterArgs a) {
       }
       ow.put(e, a0, a1);
     }
-    ow.report(a);
+    ow.report(a, jp);
     return;
   }
   if (FMT == FMT_ROWPAIR) {
@@ -1079,7 +1079,7 @@ __device__ __forceinline__ void filter_p2_body(const FilterArgs &a, const int jp
       if (!has1) z.y = 0.0f;
       ow.put(e, z.x, z.y);
     }
-    ow.report(a);
+    ow.report(a, jp);
     return;
   }
   // the other formats take a sample and the next: a warp takes 31 consecutive elements e at a time: lane l computes the final

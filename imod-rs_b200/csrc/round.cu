@@ -211,7 +211,7 @@ int round_plan_issue(RoundPlan &p, cudaStream_t st) {
     bl.max_views = g.max_views;
     const int rc = launch_bp_group(g.group, bl, st);
     if (rc != TG_OK) return rc;
-    ++launches;
+    launches += bp_group_launches(g.group);
   }
   for (tg_session *s : p.bp_single) {
     const cudaStream_t own = s->st;

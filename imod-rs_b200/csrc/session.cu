@@ -156,7 +156,7 @@ static void free_session(tg_session *s) {
   void *ptrs[] = {s->d_raw, s->d_logd, s->d_means, s->d_vol, s->d_sino, s->d_tmp, s->d_volg, s->d_volh, s->d_maxbits, s->d_mpart, s->d_pairs,
                   s->d_part, s->d_slice_stats, s->d_stats3, s->d_vg, s->d_vg2, s->d_weights,
                   s->d_conv, s->d_stretch, s->d_tw, s->d_err, s->d_lvinfo, s->d_lgoff, s->d_lxs,
-                  s->d_lys, s->d_lgdx, s->d_lgdy, s->d_ltab, s->d_xtb, s->d_lbnd, s->d_half, s->d_tmap};
+                  s->d_lys, s->d_lgdx, s->d_lgdy, s->d_ltab, s->d_xtb, s->d_lbnd, s->d_half, s->d_tmap, s->d_flags};
   for (void *p : ptrs)
     if (p) cudaFree(p);
   for (auto &e : s->ev)
@@ -170,7 +170,7 @@ void free_session_async(tg_session *s, cudaStream_t after) {
   void *ptrs[] = {s->d_raw, s->d_logd, s->d_means, s->d_vol, s->d_sino, s->d_tmp, s->d_volg, s->d_volh, s->d_maxbits, s->d_mpart, s->d_pairs,
                   s->d_part, s->d_slice_stats, s->d_stats3, s->d_vg, s->d_vg2, s->d_weights,
                   s->d_conv, s->d_stretch, s->d_tw, s->d_err, s->d_lvinfo, s->d_lgoff, s->d_lxs,
-                  s->d_lys, s->d_lgdx, s->d_lgdy, s->d_ltab, s->d_xtb, s->d_lbnd, s->d_half, s->d_tmap};
+                  s->d_lys, s->d_lgdx, s->d_lgdy, s->d_ltab, s->d_xtb, s->d_lbnd, s->d_half, s->d_tmap, s->d_flags};
   for (void *p : ptrs)
     if (p) cudaFreeAsync(p, after);
   for (auto &e : s->ev)
@@ -286,7 +286,7 @@ BpArgs bp_args(tg_session *s, int mode) {
   a.loc = local_dev(s);
   a.wait_limit_ns = s->wait_limit_ns;
   a.fault_skip_stage = s->fault_skip_stage;
-  a.nonfinite = s->d_err + 1;
+  a.flags = s->d_flags;
   a.range = reinterpret_cast<unsigned *>(s->d_err + 2);
   a.gain = s->oct_gain;
   a.tmap = s->d_tmap;
@@ -318,7 +318,7 @@ FilterArgs filter_args(tg_session *s, bool residual) {
   f.inv_n = 1.0f / (float)s->nx;
   f.plan = s->plan;
   f.err = s->d_err;
-  f.nonfinite = s->d_err + 1;
+  f.flags = s->d_flags;
   f.range = reinterpret_cast<unsigned *>(s->d_err + 2);
   f.gain = s->oct_gain;
   return f;
@@ -429,10 +429,14 @@ FpArgs fp_args(tg_session *s) {
   return f;
 }
 
-// log10 and per-view means (main.rs:608-623).  On the tensor-core path the error words
-// behind the first start over: d_err[1] is FilterArgs::nonfinite, d_err[2] its range.
+// log10 and per-view means (main.rs:608-623).  On the tensor-core path FilterArgs::flags and
+// its range (d_err[2]) start over.
+static size_t oct_flags_bytes(const tg_session *s) { return ((size_t)(s->ny + 7) / 8 + 1) * 4; }
 static int stage_log_means(tg_session *s) {
-  if (s->mma_steps) TG_CUDA(cudaMemsetAsync(s->d_err + 1, 0, 8, s->st));
+  if (s->mma_steps) {
+    TG_CUDA(cudaMemsetAsync(s->d_err + 2, 0, 4, s->st));
+    TG_CUDA(cudaMemsetAsync(s->d_flags, 0, oct_flags_bytes(s), s->st));
+  }
   launch_log_means(s->d_raw, s->d_logd, s->nx * s->ny, s->nz, s->d_mpart, s->means_pinned ? nullptr : s->d_means,
                    s->mma_steps ? reinterpret_cast<unsigned *>(s->d_err + 2) : nullptr, s->st);
   return TG_OK;
@@ -721,7 +725,8 @@ int tg::session_create_ex(const tg_geometry *g, const tg_options *opt, cudaMemPo
       (rc = dalloc(s, &s->d_tw, ((size_t)s->nx + std::max(s->nx, s->fft_n)) * 8)) ||
       (rc = dalloc(s, &s->d_stretch, (size_t)s->nviews * 4)) || (rc = dalloc(s, &s->d_err, 16)))
     return fail(rc);
-  if (s->mma_steps && (rc = dalloc(s, &s->d_tmap, 128))) return fail(rc);
+  if (s->mma_steps && ((rc = dalloc(s, &s->d_tmap, 128)) || (rc = dalloc(s, &s->d_flags, oct_flags_bytes(s)))))
+    return fail(rc);
   if (opt->log_transform && (rc = dalloc(s, &s->d_logd, nproj * 4))) return fail(rc);
   if (!opt->gpu_compat && opt->sirt_iters > 0 && (rc = dalloc(s, &s->d_sino, nproj * 4))) return fail(rc);
   if (!opt->gpu_compat && opt->fake_sirt > 0 && (rc = dalloc(s, &s->d_tmp, nvol * 4))) return fail(rc);

@@ -22,6 +22,7 @@ struct tg_session {  // one tilt series resident on a device
   int mma_steps = 0;       // fast or row-sum path on the tensor-core back-projector: its K steps (else 0)
   tg::TensorMap tmap{};    // TMA map of d_pairs on that path, and its copy for batched launches
   void *d_tmap = nullptr;
+  int *d_flags = nullptr;  // FilterArgs::flags on that path
   float oct_gain = 1.0f;   // oct_scale's gain on that path
   float *xtb = nullptr;    // row sums (d_xtb, or the reprojector's FP32 copy, which is dead then)
   float *d_xtb = nullptr;
@@ -92,7 +93,7 @@ BpArgs bp_args(tg_session *s, int mode);
 FilterArgs filter_args(tg_session *s, bool residual);
 FpArgs fp_args(tg_session *s);
 int launch_bp(tg_session *s, int mode, int *ntiles);
-inline int bp_launch_count(const tg_session *s) { return s->xt_split ? 2 : 1; }
+inline int bp_launch_count(const tg_session *s) { return (s->xt_split ? 2 : 1) + (s->mma_steps ? 1 : 0); }
 // position form of the fast kernel: 2 with x-tilt (row sums), else whether z-factors apply
 inline int fast_zf(const tg_session *s) { return s->xt_split ? 2 : s->zf_any ? 1 : 0; }
 // Series whose back-projections share a batched launch: the fast kernel's by z-factor and
@@ -104,6 +105,7 @@ inline BpGroup bp_group(const tg_session *s) {
 }
 // fills a's tile grid for its group's kernel; returns its tiles
 long long bp_group_tiles(const BpGroup &g, BpArgs &a);
+inline int bp_group_launches(const BpGroup &g) { return std::get<2>(g) < 0 ? 2 : 1; }
 int launch_bp_group(const BpGroup &g, const BatchLaunch &bl, cudaStream_t st);
 int autotune(tg_session *s);
 // the tile variant already tuned for this shape (or pinned by TG_BP_VARIANT), else -1

@@ -95,7 +95,7 @@ struct FilterArgs {
   float inv_n;
   FftPlanDev plan;
   int *err;                 // session error word: bit 2 set when a value exceeds the FP16 range
-  int *nonfinite;           // OCT: set to 1 when a staged value is infinite or NaN
+  int *flags;               // OCT, per block of 8 rows: 1 where a staged value is infinite or NaN; then 1 if any is
   const unsigned *range;    // OCT: see oct_scale
   float gain;
 };
@@ -154,9 +154,9 @@ struct BpArgs {
   // stage of each tile, so the consumers' wait on it runs out; -1: none
   int fault_skip_stage;
   // tensor-core kernel: slices per tile (set by bp_mma_plan), and this pass's
-  // FilterArgs::nonfinite, range and gain
+  // FilterArgs::flags, range and gain
   int nper;
-  const int *nonfinite;
+  const int *flags;
   const unsigned *range;
   const void *tmap;         // batched launches: the series' TensorMap, in device memory
   float gain;

@@ -114,3 +114,53 @@ def test_bounded_wait_in_a_batch():
     b.close()
     for s in ss:
         s.close()
+
+
+# ---- values that are not finite: the blocks of 8 slices that hold them, and no other ----
+
+@pytest.mark.parametrize("bad", [np.nan, np.inf, -np.inf])
+def test_a_bad_sample_leaves_the_other_blocks_as_they_were(bad):
+    ang = angles(-60, 60, 12)
+    proj = smooth_stack(len(ang), 37, 90, seed=4)
+    kw = dict(thickness=44, fill_mode="zero")
+    with session(90, 37, ang, proj, **kw) as s:
+        s.reconstruct()
+        good, _ = s.download()
+        proj[2, 11, 40] = proj[5, 36, 3] = bad
+        s.upload(proj)
+        s.reconstruct()
+        vol, _ = s.download()
+        blocks = np.r_[8:16, 32:37]
+        np.testing.assert_array_equal(np.delete(vol, blocks, 0), np.delete(good, blocks, 0))
+        assert np.isnan(vol[11]).any() and np.isnan(vol[36]).any()
+        rest = np.r_[8:10, 12:16, 32:36]
+        assert rel_l2(vol[rest], good[rest]) <= TOL
+        proj = smooth_stack(len(ang), 37, 90, seed=4)
+        s.upload(proj)
+        s.reconstruct()
+        np.testing.assert_array_equal(s.download()[0], good)
+
+
+@pytest.mark.parametrize("sirt", [0, 1])
+def test_a_series_full_of_bad_rows_does_not_hold_up_the_next_one(sirt):
+    # in one batched launch the good series' tiles follow the bad one's in every block; its
+    # waits are shorter than the bad one's tiles of a block together
+    nb, ng = 61, 20
+    angb, angg = np.linspace(-60, 60, nb).astype(np.float32), np.linspace(-60, 60, ng).astype(np.float32)
+    kw = dict(fill_mode="zero", sirt=sirt, sirt_relax=0.5)
+    bad = smooth_stack(nb, 256, 300, seed=1)
+    bad[0, ::2, 7] = np.nan
+    good = smooth_stack(ng, 40, 200, seed=2)
+    with session(200, 40, angg, good, thickness=300, **kw) as g:
+        g.reconstruct()
+        want, _ = g.download()
+        with session(300, 256, angb, bad, thickness=300, **kw) as s:
+            b = T.Batch()
+            b.add(s)
+            b.add(g)
+            g.inject_wait_fault(-1, 20000)
+            s.inject_wait_fault(-1, 20000)
+            b.reconstruct()
+            np.testing.assert_array_equal(g.download()[0], want)
+            assert np.isnan(s.download()[0]).any(axis=(1, 2)).all()
+            b.close()
