@@ -25,7 +25,9 @@
 // Persistent CTAs (one per SM), warp-specialised, all roles walking the same tiles:
 //   warps 0-7   consumers: tensor memory -> registers, epilogue.  128 accumulators
 //               per thread: one voxel x 128 slices.
-//   warps 8-11  weights: one voxel per thread, its rows of W per view to shared memory
+//   warps 8-11  weights: one voxel per thread, its rows of W per view to shared memory; and
+//               the sum of the means of the views whose rows the voxel is outside of,
+//               which the consumers add to its slices (it is the same in all of them)
 //   warp 12     producer: one TMA box per view, the 16-element windows of the tile's
 //               8-slice blocks in both planes (layout OCT: [plane][view][block of 8
 //               slices][element][8]); any start element, since an element is 16 bytes
@@ -87,8 +89,9 @@ template <int KS> struct Cfg {
   static constexpr int STAGE = 2 * VIEW;             // a ring stage is a pair of views
   static constexpr int TR = NCONS * 16 * 33 * 4;     // statistics transpose
   static constexpr int PART = MAX_N * 4 * 16;        // statistics of the four lane quarters
+  static constexpr int FILL = 2 * 128 * 4;           // fill sums of the voxels of two tiles
   static constexpr int NST = KS == 1 ? 4 : 2;
-  static constexpr int SMEM = NST * STAGE + TR + PART;
+  static constexpr int SMEM = NST * STAGE + TR + PART + FILL;
   static_assert(SMEM <= 226 * 1024 && SMEM > 114 * 1024, "one CTA per SM");
 };
 
@@ -152,10 +155,12 @@ __device__ __forceinline__ void accumulate(float (&acc)[128], int c, const float
   }
 }
 
-// The samples of a voxel in 8 slices summed over the views without the tensor cores
-__device__ __forceinline__ void sum_views(const BpArgs &a, float dx, float dz, int blk, float (&s8)[8]) {
+// The samples of a voxel in 8 slices, and apart from them its fills, summed over the views
+// without the tensor cores
+__device__ __forceinline__ void sum_views(const BpArgs &a, float dx, float dz, int blk, float (&s8)[8], float &fill) {
 #pragma unroll
   for (int j = 0; j < 8; ++j) s8[j] = 0.0f;
+  fill = 0.0f;
   const size_t plane = (size_t)a.nviews * a.rows_alloc * a.PW;
   auto value = [](uint32_t hi, uint32_t lo, int i) {
     const float h = half_val(hi, i);
@@ -169,6 +174,7 @@ __device__ __forceinline__ void sum_views(const BpArgs &a, float dx, float dz, i
     int k = (int)(__float_as_uint(tt) - MAGIC_BITS);
     const bool in = (uint32_t)k <= (uint32_t)(a.nx - 2);
     if (!in && k >= 0) ++k;
+    if (!in && a.fill) fill = __fadd_rn(fill, __ldg(a.fill + v));
     const uint4 *e = reinterpret_cast<const uint4 *>(a.pairs) + ((size_t)v * a.rows_alloc + blk) * a.PW + (k + a.padL);
     const uint4 u0 = __ldg(e), z0 = __ldg(e + plane), u1 = in ? __ldg(e + 1) : u0, z1 = in ? __ldg(e + 1 + plane) : z0;
     const uint32_t *p0 = &u0.x, *q0 = &z0.x, *p1 = &u1.x, *q1 = &z1.x;
@@ -214,11 +220,12 @@ template <int KS, class Job>
 __device__ __forceinline__ void mma_body(const Job &job, int ntiles, unsigned char *sm) {
   using C = Cfg<KS>;
   constexpr int KW = C::KW, NST = C::NST;
-  __shared__ __align__(8) uint64_t fullb[NST], full[NST], empty[NST], tfull[2], tempty[2], done[2];
+  __shared__ __align__(8) uint64_t fullb[NST], full[NST], empty[NST], tfull[2], tempty[2], ffull[2], fempty[2], done[2];
   __shared__ uint32_t s_tmem;
   __shared__ volatile int s_abort;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const uint32_t ring = smem_u32(sm);
+  float *fills = reinterpret_cast<float *>(sm + NST * C::STAGE + C::TR + C::PART);
 
   if (warp == 13) tmem_alloc(smem_u32(&s_tmem), 512);
   if (tid == 0) {
@@ -230,6 +237,8 @@ __device__ __forceinline__ void mma_body(const Job &job, int ntiles, unsigned ch
     for (int b = 0; b < 2; ++b) {
       mbar_init(smem_u32(&tfull[b]), 1);
       mbar_init(smem_u32(&tempty[b]), NCONS);
+      mbar_init(smem_u32(&ffull[b]), NWGT);
+      mbar_init(smem_u32(&fempty[b]), NCONS);
     }
     for (int e = 0; e < 2; ++e) mbar_init(smem_u32(&done[e]), 1);
     fence_mbar_init();
@@ -248,6 +257,7 @@ __device__ __forceinline__ void mma_body(const Job &job, int ntiles, unsigned ch
     float *tr = reinterpret_cast<float *>(sm + NST * C::STAGE) + warp * (16 * 33);
     StatPartial *part = reinterpret_cast<StatPartial *>(sm + NST * C::STAGE + C::TR);
     int ph = 0;  // bit e: phase of tensor-memory buffer e
+    int fb = 0, fph = 0;  // the tile's buffer of fill sums and its phase
     for (int t0 = blockIdx.x; t0 < ntiles; t0 += gridDim.x) {
       int t = t0;
       const BpArgs &a = job(t);
@@ -282,6 +292,12 @@ __device__ __forceinline__ void mma_body(const Job &job, int ntiles, unsigned ch
         if (cnt == 0 && lane == 0) mbar_arrive(smem_u32(&tempty[e]));
         ph ^= 1 << e;
       }
+      go = go && warp_poll(smem_u32(&ffull[fb]), fph, &s_abort, limit);
+      const float fill = fills[fb * 128 + (warp & 3) * 32 + lane];
+      __syncwarp();
+      if (lane == 0) mbar_arrive(smem_u32(&fempty[fb]));
+      fph ^= fb;
+      fb ^= 1;
       if (!go) s_abort = 1;
       // all consumer warps store this tile, or none does: the barriers of the epilogue expect
       // them all.  (Behind this one, the previous tile's statistics have been read.)
@@ -296,7 +312,7 @@ __device__ __forceinline__ void mma_body(const Job &job, int ntiles, unsigned ch
       {  // undo the staging scale (a power of two)
         const float inv = oct_scale(a.range, a.gain, true);
 #pragma unroll
-        for (int i = 0; i < 128; ++i) acc[i] = __fmul_rn(acc[i], inv);
+        for (int i = 0; i < 128; ++i) acc[i] = fmaf(acc[i], inv, fill);
       }
       const int iy = q.iy0 + c0, ny = min(cnt, a.ny - iy);  // slices of this warp inside the volume
       // its blocks of 8 slices that hold a value that is not finite: bp_oct_kernel stores those
@@ -383,7 +399,7 @@ __device__ __forceinline__ void mma_body(const Job &job, int ntiles, unsigned ch
     reg_dec<REG_WGT>();
     const int row = tid - NCONS * 32;
     const int2 vox = hex_voxel(min(row, NVOX - 1));
-    int b = 0, ph = 1;
+    int b = 0, ph = 1, fb = 0, fph = 1;
     for (int t0 = blockIdx.x; t0 < ntiles && !__any_sync(0xffffffffu, s_abort); t0 += gridDim.x) {
       int t = t0;
       const BpArgs &a = job(t);
@@ -393,12 +409,14 @@ __device__ __forceinline__ void mma_body(const Job &job, int ntiles, unsigned ch
       const bool ok = row < NVOX && ox >= 0 && ox < a.onx && oz >= 0 && oz < a.onz;
       const float dx = __fsub_rn((float)ox, a.ocx), dz = __fsub_rn((float)oz, a.cz), cx = a.cx;
       const float4 *vg = a.vg;
+      const float *means = a.fill;
+      float fill = 0.0f;
       const uint64_t limit = a.wait_limit_ns;
       int k0s = 0;
       // a voxel's row of W in view v: p the words at element pair kw and the next in the
       // first block, r in the second
       struct Row { uint32_t p0, p1, r0, r1; int kw; };
-      auto row_of = [&](const float4 &g, int k0) -> Row {
+      auto row_of = [&](const float4 &g, int k0, int v) -> Row {
         const float x = position(dx, dz, g, cx);
         const float tt = __fadd_rd(x, MAGIC);  // MAGIC + floor(x), exactly
         const float f = __fsub_rn(x, __fsub_rn(tt, MAGIC));
@@ -408,8 +426,9 @@ __device__ __forceinline__ void mma_body(const Job &job, int ntiles, unsigned ch
         uint32_t w0 = half_pair(omf, f);
         uint32_t w1 = half_pair(__fsub_rn(omf, half_val(w0, 0)), __fsub_rn(f, half_val(w0, 1)));
         if ((uint32_t)k > (uint32_t)nx2) {
-          // outside the row: the fill alone, which the padding holds (element nx - 1 is the
-          // last sample, so the right side takes the element after)
+          // outside the row: the fill alone, which the padding holds in edge mode (element nx - 1
+          // is the last sample, so the right side takes the element after)
+          if (means && v < nviews) fill = __fadd_rn(fill, __ldg(means + v));
           w0 = half_pair(1.0f, 0.0f);
           w1 = 0u;
           k += k >= 0 ? 1 : 0;
@@ -438,7 +457,7 @@ __device__ __forceinline__ void mma_body(const Job &job, int ntiles, unsigned ch
       for (int v = 0; v < nviews; v += 2) {
         if ((v & 31) == 0) k0s = window_start<KW>(a, q, v + lane);
         const int ka = __shfl_sync(0xffffffffu, k0s, v & 31), kb = __shfl_sync(0xffffffffu, k0s, (v + 1) & 31);
-        const Row wa = row_of(g0, ka), wb = row_of(g1, kb);
+        const Row wa = row_of(g0, ka, v), wb = row_of(g1, kb, v + 1);
         g0 = __ldg(vg + min(v + 2, nviews - 1));
         g1 = __ldg(vg + min(v + 3, nviews - 1));
         const bool two = v + 1 < nviews;
@@ -452,6 +471,13 @@ __device__ __forceinline__ void mma_body(const Job &job, int ntiles, unsigned ch
         __syncwarp();
         if (lane == 0) mbar_arrive(smem_u32(&full[b]));
         if (++b == NST) { b = 0; ph ^= 1; }
+      }
+      if (go && (go = warp_poll(smem_u32(&fempty[fb]), fph, &s_abort, limit))) {
+        fills[fb * 128 + row] = fill;
+        __syncwarp();
+        if (lane == 0) mbar_arrive(smem_u32(&ffull[fb]));
+        fph ^= fb;
+        fb ^= 1;
       }
       if (!go) {
         s_abort = 1;
@@ -638,14 +664,14 @@ __device__ __forceinline__ void oct_blocks(const BpArgs &a, int ntiles_xz) {
         const bool ok = tid < NVOX && ox >= 0 && ox < a.onx && oz >= 0 && oz < a.onz;
         const float dx = __fsub_rn((float)min(max(ox, 0), a.onx - 1), a.ocx);
         const float dz = __fsub_rn((float)min(max(oz, 0), a.onz - 1), a.cz);
-        float s8[8];
-        sum_views(a, dx, dz, blk, s8);
+        float s8[8], fill;
+        sum_views(a, dx, dz, blk, s8, fill);
         float *out = a.vol + ((size_t)iy * a.onz + oz) * a.onx + ox;
         const size_t sl = (size_t)a.onz * a.onx;
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
           const bool put = ok && iy + j < a.ny;
-          float y = __fmul_rn(__fmul_rn(s8[j], inv), a.inv_n);
+          float y = __fmul_rn(fmaf(s8[j], inv, fill), a.inv_n);
           if (a.mode == 2 && put) y = __fadd_rn(out[j * sl], __fmul_rn(a.relax, y));
           if (a.mode == 0) {
             y = __fadd_rn(__fmul_rn(__fmul_rn(y, a.dw), a.os), a.oa);

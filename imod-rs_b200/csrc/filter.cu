@@ -475,7 +475,7 @@ __global__ void __launch_bounds__(256) filter_kernel(FilterArgs a) {
     row0 = s0;
     row1 = s1;
   }
-  const float fillv = a.fill ? a.fill[v] : 0.0f;
+  const float fillv = FMT != FMT_OCT && a.fill ? a.fill[v] : 0.0f;
   float hmax = 0.0f;  // largest |value| packed into FP16 by this thread
   if (FMT == FMT_ROWS) {  // plain filtered rows written back over the input rows
     float *o0 = reinterpret_cast<float *>(a.out) + ((size_t)v * a.ny + r0) * n;
@@ -1064,7 +1064,7 @@ __device__ __forceinline__ void filter_p2_body(const FilterArgs &a, const int jp
     return make_float2(0.0f, 0.0f);
   };
   // pack into the staging format with the reference's fill rule (main.rs:386-406)
-  const float fillv = a.fill ? a.fill[v] : 0.0f;
+  const float fillv = FMT != FMT_OCT && a.fill ? a.fill[v] : 0.0f;
   auto fill = [&](int k) -> float2 {
     if (a.fill_mode == TG_FILL_ZERO) return make_float2(0.0f, 0.0f);
     if (a.fill_mode == TG_FILL_EDGE) return fin(k < 0 ? 0 : n - 1);

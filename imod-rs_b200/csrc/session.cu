@@ -286,6 +286,7 @@ BpArgs bp_args(tg_session *s, int mode) {
   a.loc = local_dev(s);
   a.wait_limit_ns = s->wait_limit_ns;
   a.fault_skip_stage = s->fault_skip_stage;
+  a.fill = !s->o.gpu_compat && s->o.fill_mode == TG_FILL_MEAN ? s->d_means : nullptr;
   a.flags = s->d_flags;
   a.range = reinterpret_cast<unsigned *>(s->d_err + 2);
   a.gain = s->oct_gain;

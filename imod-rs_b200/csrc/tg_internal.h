@@ -25,7 +25,8 @@ namespace tg {
 // FP32 float2 (a, b), FP16/BF16 uint32 h2(a, d).
 // OCT is FP32 staging for the tensor-core back-projector: 8 consecutive rows per
 // element, [plane][view][block of 8 rows][PW][8] halves; planes 0 and 1 hold the FP16
-// leading part and remainder of row[k] * oct_scale, k outside [0, nx) the fill's.
+// leading part and remainder of row[k] * oct_scale, k outside [0, nx) the edge sample's or 0
+// (a view's mean need not fit the rows' scale: the back-projector adds it itself, BpArgs::fill).
 enum Fmt { FMT_ROWPAIR = 0, FMT_SINGLE = 1, FMT_ROWS = 2 /* plain filtered rows, in place */, FMT_OCT = 3 };
 
 inline int elem_bytes(int fmt, int store) {
@@ -156,6 +157,7 @@ struct BpArgs {
   // tensor-core kernel: slices per tile (set by bp_mma_plan), and this pass's
   // FilterArgs::flags, range and gain
   int nper;
+  const float *fill;        // mean mode: value of a view's samples outside its rows, else nullptr
   const int *flags;
   const unsigned *range;
   const void *tmap;         // batched launches: the series' TensorMap, in device memory

@@ -164,3 +164,66 @@ def test_a_series_full_of_bad_rows_does_not_hold_up_the_next_one(sirt):
             np.testing.assert_array_equal(g.download()[0], want)
             assert np.isnan(s.download()[0]).any(axis=(1, 2)).all()
             b.close()
+
+
+# ---- mean fill: a view's mean is not bound to the range of the rows that are staged ----
+
+def both(monkeypatch, run):
+    out = []
+    for v in (SHARED, TENSOR):
+        monkeypatch.setenv("TG_BP_VARIANT", v)
+        out.append(run())
+    return out
+
+
+@pytest.mark.parametrize("top,mean", [(10.0, 5000.0), (1e-3, 4.0), (0.0, 70000.0), (0.0, 1e-20), (1e6, 1e-6), (1.0, -3e30)])
+def test_dark_slab_of_a_bright_series(top, mean, monkeypatch):
+    ang = angles(-60, 60, 10)
+    proj = (top * smooth_stack(len(ang), 20, 64, seed=3)).astype(np.float32)
+    means = (mean * np.linspace(0.5, 1.5, len(ang))).astype(np.float32)
+
+    def run():  # wide enough that voxels project outside the rows
+        with session(64, 20, ang, proj, width=90, thickness=50) as s:
+            s.set_view_means(means)
+            s.reconstruct()
+            return s.download()
+    (want, wst), (got, st) = both(monkeypatch, run)
+    assert np.isfinite(want).all() and np.isfinite(got).all()
+    assert rel_l2(got, want) <= TOL
+    assert st["amin"] == pytest.approx(wst["amin"], rel=1e-5) and st["amax"] == pytest.approx(wst["amax"], rel=1e-5)
+
+
+def test_residuals_far_below_the_means(monkeypatch):
+    # an empty volume stays empty where the projections are a millionth of their pinned means
+    ang = angles(-60, 60, 8)
+    proj = smooth_stack(len(ang), 20, 64, seed=6)
+
+    def run():
+        with session(64, 20, ang, proj, width=90, thickness=50, sirt=3, sirt_relax=0.1) as s:
+            s.set_view_means(np.full(len(ang), 3e6, np.float32))
+            s.sirt_restore(np.zeros(s.out_shape, np.float32), 0)
+            s.sirt_iterate(3)
+            s.sirt_end()
+            return s.download()[0]
+    want, got = both(monkeypatch, run)
+    assert np.isfinite(got).all()
+    assert rel_l2(got, want) <= TOL
+
+
+@pytest.mark.parametrize("bad", [np.nan, np.inf])
+def test_bad_samples_with_mean_fill(bad, monkeypatch):
+    # the view's mean is not finite either: every voxel outside that view's rows takes it, and
+    # those inside keep the values of their own rows
+    ang = angles(-60, 60, 12)
+    proj = smooth_stack(len(ang), 37, 90, seed=4)
+    proj[9, 11, 40] = bad
+
+    def run():
+        with session(90, 37, ang, proj, width=120, thickness=60) as s:
+            s.reconstruct()
+            return s.download()[0]
+    want, got = both(monkeypatch, run)
+    np.testing.assert_array_equal(np.isfinite(got), np.isfinite(want))
+    good = np.isfinite(want)
+    assert good.any() and not good[0].all()
+    assert rel_l2(got[good], want[good]) <= TOL
