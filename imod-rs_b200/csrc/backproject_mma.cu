@@ -12,8 +12,8 @@
 // 128 voxels x N = 256 slices per term.  (An 8 x 16 rectangle needs up to 19, so two.)
 //
 // FP32 from FP16 operands: rows = hi + lo and weights = hi + lo in FP16 (22 significant
-// bits), three products hi*lo + lo*hi + hi*hi; rows are staged times a power of two
-// that keeps them in FP16's range (oct_scale), undone on the sums.  The tensor cores
+// bits), three products hi*lo + lo*hi + hi*hi; each block of 8 rows is staged times a power
+// of two that keeps it in FP16's range (oct_exponent), undone on the sums.  The tensor cores
 // truncate their FP32 sums, so they form the samples of two views only (their small
 // terms first), and the sum over views is the consumer warps': tensor memory -> FP32
 // register accumulators, round to nearest.  The result is as close to FP64 as the
@@ -35,8 +35,8 @@
 //               and plane instead: 62 cycles each, 64 a view, measured 4x slower.)
 //   warps 13-14 one thread each issues the tcgen05.mma's of every other view into its
 //               tensor-memory buffer of 256 columns and commits
-// A tile's epilogue overlaps the next tile's first views.  Blocks of slices with values
-// that are not finite take bp_oct_kernel, launched behind it.
+// A tile's epilogue overlaps the next tile's first views.  Blocks of 8 slices with values
+// that are not finite, or rows far below their scale, take bp_oct_kernel, launched behind it.
 #include <cuda.h>
 #include <cuda_fp16.h>
 
@@ -156,7 +156,7 @@ __device__ __forceinline__ void accumulate(float (&acc)[128], int c, const float
 }
 
 // The samples of a voxel in 8 slices, and apart from them its fills, summed over the views
-// without the tensor cores
+// without the tensor cores, each row unscaled by its own exponent
 __device__ __forceinline__ void sum_views(const BpArgs &a, float dx, float dz, int blk, float (&s8)[8], float &fill) {
 #pragma unroll
   for (int j = 0; j < 8; ++j) s8[j] = 0.0f;
@@ -176,12 +176,14 @@ __device__ __forceinline__ void sum_views(const BpArgs &a, float dx, float dz, i
     if (!in && k >= 0) ++k;
     if (!in && a.fill) fill = __fadd_rn(fill, __ldg(a.fill + v));
     const uint4 *e = reinterpret_cast<const uint4 *>(a.pairs) + ((size_t)v * a.rows_alloc + blk) * a.PW + (k + a.padL);
+    const uint2 exps = __ldg(reinterpret_cast<const uint2 *>(a.exps) + (size_t)v * ((a.ny + 7) / 8) + blk);
     const uint4 u0 = __ldg(e), z0 = __ldg(e + plane), u1 = in ? __ldg(e + 1) : u0, z1 = in ? __ldg(e + 1 + plane) : z0;
     const uint32_t *p0 = &u0.x, *q0 = &z0.x, *p1 = &u1.x, *q1 = &z1.x;
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
+      const float inv = pow2f(-(int)(signed char)((j < 4 ? exps.x : exps.y) >> (8 * (j & 3))));
       const float v0 = value(p0[j / 2], q0[j / 2], j & 1);
-      s8[j] += in ? v0 * (1.0f - f) + value(p1[j / 2], q1[j / 2], j & 1) * f : v0;
+      s8[j] += inv * (in ? v0 * (1.0f - f) + value(p1[j / 2], q1[j / 2], j & 1) * f : v0);
     }
   }
 }
@@ -309,14 +311,19 @@ __device__ __forceinline__ void mma_body(const Job &job, int ntiles, unsigned ch
       // ---------------- epilogue ----------------
       const size_t sl = (size_t)onz * onx;
       const float inv_n = a.inv_n;
-      {  // undo the staging scale (a power of two)
-        const float inv = oct_scale(a.range, a.gain, true);
-#pragma unroll
-        for (int i = 0; i < 128; ++i) acc[i] = fmaf(acc[i], inv, fill);
-      }
       const int iy = q.iy0 + c0, ny = min(cnt, a.ny - iy);  // slices of this warp inside the volume
-      // its blocks of 8 slices that hold a value that is not finite: bp_oct_kernel stores those
-      const unsigned skip = __ballot_sync(0xffffffffu, 8 * lane < ny && __ldg(a.flags + min(iy / 8 + lane, (a.ny - 1) / 8)));
+      // its blocks of 8 slices that bp_oct_kernel stores
+      const int blk = min(iy / 8 + lane, (a.ny - 1) / 8);
+      const unsigned skip = __ballot_sync(0xffffffffu, 8 * lane < ny && __ldg(a.flags + blk));
+      {  // undo the blocks' staging scales (powers of two)
+        const float inv = pow2f(-oct_exponent(__uint_as_float(__ldg(a.range + blk)), a.gain));
+#pragma unroll
+        for (int b = 0; b < 16; ++b) {
+          const float u = __shfl_sync(0xffffffffu, inv, b);
+#pragma unroll
+          for (int j = 0; j < 8; ++j) acc[8 * b + j] = fmaf(acc[8 * b + j], u, fill);
+        }
+      }
       float *out = a.vol + ((size_t)iy * onz + oz) * onx + ox;
       const int mode = a.mode;
       if (mode == 2) {  // SIRT update vol += relax * v: 8 old values loaded together before their stores
@@ -639,9 +646,10 @@ __global__ void __launch_bounds__(NTHR, 1) bp_mma_batch_kernel(const BpArgs *__r
   mma_body<KS>(ManyJobs{jobs, njobs}, ntiles, sm);
 }
 
-// The blocks of 8 slices that hold a value that is not finite, which a product with the zeros of
-// W spreads to the voxels of its slice that do not sample it: the same tiles, one voxel
-// per thread, sample by sample.  A kernel of its own, so that the tensor-core kernel's warps
+// The blocks of 8 slices that the tensor-core kernel leaves out: those with rows of a scale of
+// their own, and with a value that is not finite, which a product with the zeros of W spreads
+// to the voxels of its slice that do not sample it.  The same tiles, one voxel per thread, sample
+// by sample.  A kernel of its own, so that the tensor-core kernel's warps
 // never wait for such a tile and the rest of a series keeps its speed; with no such block a
 // CTA reads one word and ends.
 constexpr int OCT_T = 128;
@@ -651,7 +659,6 @@ __device__ __forceinline__ void oct_blocks(const BpArgs &a, int ntiles_xz) {
   __shared__ StatPartial part[OCT_T / 32][8];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int2 vox = hex_voxel(min(tid, NVOX - 1));
-  const float inv = oct_scale(a.range, a.gain, true);
   int first = blockIdx.x;  // this CTA's first tile of the next flagged block
   for (int b0 = 0; b0 < nblk; b0 += 32) {
     unsigned todo = __ballot_sync(0xffffffffu, b0 + lane < nblk && a.flags[min(b0 + lane, nblk - 1)]);
@@ -671,7 +678,7 @@ __device__ __forceinline__ void oct_blocks(const BpArgs &a, int ntiles_xz) {
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
           const bool put = ok && iy + j < a.ny;
-          float y = __fmul_rn(fmaf(s8[j], inv, fill), a.inv_n);
+          float y = __fmul_rn(__fadd_rn(s8[j], fill), a.inv_n);
           if (a.mode == 2 && put) y = __fadd_rn(out[j * sl], __fmul_rn(a.relax, y));
           if (a.mode == 0) {
             y = __fadd_rn(__fmul_rn(__fmul_rn(y, a.dw), a.os), a.oa);

@@ -115,17 +115,45 @@ __device__ __forceinline__ float finite_abs(float x) { return fabsf(x) <= 3.4028
 __device__ __forceinline__ float finite_abs4(float4 v) {
   return fmaxf(fmaxf(finite_abs(v.x), finite_abs(v.y)), fmaxf(finite_abs(v.z), finite_abs(v.w)));
 }
-// raises *range to the block's largest mx (nonnegative floats order as their bits)
-__device__ __forceinline__ void raise_range(float mx, unsigned *range) {
-  const unsigned m = __reduce_max_sync(0xffffffffu, __float_as_uint(mx));
-  if ((threadIdx.x & 31) == 0 && m) atomicMax(range, m);
-}
+// (nonnegative floats order as their bits)
+__device__ __forceinline__ unsigned warp_max(float mx) { return __reduce_max_sync(0xffffffffu, __float_as_uint(mx)); }
+
+// Largest magnitudes per block of 8 rows over one chunk of a view's pixels.  A thread meets
+// the pixels in rising order: it keeps the maximum of the block it is in and hands it over
+// when it leaves the block (a 16-byte group on the border counts for both).
+struct RangeTracker {
+  static constexpr int MAX = 65536 / 8 / MEAN_CH + 2;  // blocks that a chunk touches, at most
+  unsigned *blk;                                       // [MAX] in shared memory, zero
+  int size, end, b = 0;                                // pixels of a block; end of block b, from the chunk's start
+  float mx = 0.0f;
+  __device__ RangeTracker(unsigned *blk, int nx, long c0) : blk(blk), size(8 * nx), end(size - (int)(c0 % size)) {}
+  __device__ __forceinline__ void flush() {
+    const unsigned m = __float_as_uint(mx);
+    if (m > blk[b]) atomicMax(&blk[b], m);
+  }
+  __device__ __forceinline__ void note(int pos, int len, float m) {
+    if (pos + len > end) {
+      if (pos < end) mx = fmaxf(mx, m);
+      flush();
+      const int n = (pos + len - 1 - end) / size + 1;
+      b += n;
+      end += n * size;
+      mx = m;
+      return;
+    }
+    mx = fmaxf(mx, m);
+  }
+};
 
 template <bool LOG, bool RANGE>
 __global__ void __launch_bounds__(256) log_sum_kernel(const float *__restrict__ raw, float *__restrict__ logd,
-                                                      long npix, double *partials, unsigned *range) {
+                                                      long npix, double *partials, int nx, unsigned *range) {
   const int v = blockIdx.y, c = blockIdx.x;
-  float mx = 0.0f;
+  __shared__ unsigned blk[RANGE ? RangeTracker::MAX : 1];
+  if (RANGE) {
+    for (int i = threadIdx.x; i < RangeTracker::MAX; i += blockDim.x) blk[i] = 0;
+    __syncthreads();
+  }
   __shared__ LogTable lt;
   if (LOG) log_table(lt);
   const size_t base = (size_t)v * npix;
@@ -134,12 +162,14 @@ __global__ void __launch_bounds__(256) log_sum_kernel(const float *__restrict__ 
   long a0 = c0 + (long)((4 - ((base + c0) & 3)) & 3);
   if (a0 > c1) a0 = c1;
   const long a1 = a0 + ((c1 - a0) & ~3L);
+  RangeTracker rt(blk, RANGE ? nx : 1, c0);
+  const int p0 = (int)(a0 - c0);
   double s = 0.0;
   for (long i = c0 + threadIdx.x; i < a0; i += blockDim.x) {
     float x = raw[base + i];
     if (LOG) logd[base + i] = x = log_sample_fast(x, lt);
     s += (double)x;
-    if (RANGE) mx = fmaxf(mx, finite_abs(x));
+    if (RANGE) rt.note((int)(i - c0), 1, finite_abs(x));
   }
   const float4 *r4 = reinterpret_cast<const float4 *>(raw + base + a0);
   float4 *l4 = LOG ? reinterpret_cast<float4 *>(logd + base + a0) : nullptr;
@@ -155,25 +185,31 @@ __global__ void __launch_bounds__(256) log_sum_kernel(const float *__restrict__ 
     }
     s += ((double)x.x + (double)x.y) + ((double)x.z + (double)x.w);
     s += ((double)y.x + (double)y.y) + ((double)y.z + (double)y.w);
-    if (RANGE) mx = fmaxf(mx, fmaxf(finite_abs4(x), finite_abs4(y)));
+    if (RANGE) {
+      rt.note(p0 + 4 * (int)i, 4, finite_abs4(x));
+      rt.note(p0 + 4 * (int)(i + blockDim.x), 4, finite_abs4(y));
+    }
   }
   if (i < n4) {
     const float4 x = log4<LOG>(__ldcs(r4 + i), lt);
     if (LOG) l4[i] = x;
     s += ((double)x.x + (double)x.y) + ((double)x.z + (double)x.w);
-    if (RANGE) mx = fmaxf(mx, finite_abs4(x));
+    if (RANGE) rt.note(p0 + 4 * (int)i, 4, finite_abs4(x));
   }
   for (long k = a1 + threadIdx.x; k < c1; k += blockDim.x) {
     float x = raw[base + k];
     if (LOG) logd[base + k] = x = log_sample_fast(x, lt);
     s += (double)x;
-    if (RANGE) mx = fmaxf(mx, finite_abs(x));
+    if (RANGE) rt.note((int)(k - c0), 1, finite_abs(x));
   }
-  if (RANGE) raise_range(mx, range);
+  if (RANGE) rt.flush();
   __shared__ double red[8];
   for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
   if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
   __syncthreads();
+  if (RANGE)
+    for (int j = threadIdx.x; j < RangeTracker::MAX; j += blockDim.x)
+      if (blk[j]) atomicMax(range + c0 / (8 * nx) + j, blk[j]);
   if (threadIdx.x == 0) {
     double t = 0.0;
     for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += red[w];
@@ -181,27 +217,33 @@ __global__ void __launch_bounds__(256) log_sum_kernel(const float *__restrict__ 
   }
 }
 
-// largest finite |in - sub| (a SIRT residual before its filter)
+// largest finite |in - sub| (a SIRT residual before its filter) of one block of 8 rows of a
+// few views
+constexpr int RANGE_VIEWS = 4;
 __global__ void __launch_bounds__(256) residual_range_kernel(const float *__restrict__ in, const float *__restrict__ sub,
-                                                             size_t n, unsigned *range) {
-  const size_t stride = (size_t)gridDim.x * blockDim.x, n4 = n / 4;
-  const float4 *i4 = reinterpret_cast<const float4 *>(in), *s4 = reinterpret_cast<const float4 *>(sub);
+                                                             int nx, int ny, int nviews, unsigned *range) {
+  const int r0 = 8 * blockIdx.x, n = min(8, ny - r0) * nx;
   float mx = 0.0f;
-  auto diff = [](float4 a, float4 b) { return make_float4(a.x - b.x, a.y - b.y, a.z - b.z, a.w - b.w); };
-  size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  for (; i + stride < n4; i += 2 * stride) {  // four 16-byte loads in flight
-    const float4 a = __ldg(i4 + i), b = __ldg(s4 + i), c = __ldg(i4 + i + stride), d = __ldg(s4 + i + stride);
-    mx = fmaxf(mx, fmaxf(finite_abs4(diff(a, b)), finite_abs4(diff(c, d))));
+  for (int v = RANGE_VIEWS * blockIdx.y; v < min(nviews, RANGE_VIEWS * ((int)blockIdx.y + 1)); ++v) {
+    const size_t o = ((size_t)v * ny + r0) * nx;
+    const float *p = in + o, *q = sub + o;
+    const int head = min(n, (int)((4 - (o & 3)) & 3)), n4 = (n - head) / 4, tail = head + 4 * n4;
+    const float4 *p4 = reinterpret_cast<const float4 *>(p + head), *q4 = reinterpret_cast<const float4 *>(q + head);
+#pragma unroll 4
+    for (int i = threadIdx.x; i < n4; i += 256) {
+      const float4 a = __ldg(p4 + i), b = __ldg(q4 + i);
+      mx = fmaxf(mx, finite_abs4(make_float4(a.x - b.x, a.y - b.y, a.z - b.z, a.w - b.w)));
+    }
+    const int e = (int)threadIdx.x < head ? threadIdx.x : tail + (int)threadIdx.x - head;  // fewer than 8 odd samples
+    if (e < n) mx = fmaxf(mx, finite_abs(__ldg(p + e) - __ldg(q + e)));
   }
-  if (i < n4) mx = fmaxf(mx, finite_abs4(diff(__ldg(i4 + i), __ldg(s4 + i))));
-  if (blockIdx.x == 0 && threadIdx.x < n - 4 * n4)
-    mx = fmaxf(mx, finite_abs(__ldg(in + 4 * n4 + threadIdx.x) - __ldg(sub + 4 * n4 + threadIdx.x)));
-  raise_range(mx, range);
+  const unsigned m = warp_max(mx);
+  if ((threadIdx.x & 31) == 0 && m) atomicMax(range + blockIdx.x, m);
 }
 
-void launch_residual_range(const float *in, const float *sub, size_t n, unsigned *range, cudaStream_t st) {
-  const size_t nb = (n / 8 + 255) / 256;
-  residual_range_kernel<<<(unsigned)(nb < 1 ? 1 : nb > 148 * 8 ? 148 * 8 : nb), 256, 0, st>>>(in, sub, n, range);
+void launch_residual_range(const float *in, const float *sub, int nx, int ny, int nviews, unsigned *range, cudaStream_t st) {
+  const dim3 grid((ny + 7) / 8, (nviews + RANGE_VIEWS - 1) / RANGE_VIEWS);
+  residual_range_kernel<<<grid, 256, 0, st>>>(in, sub, nx, ny, nviews, range);
 }
 
 __global__ void means_final_kernel(const double *partials, long npix, int nviews, float *means) {
@@ -220,11 +262,12 @@ __global__ void view_sums_kernel(const double *partials, int nviews, double *sum
   sums[v] = t;
 }
 
-void launch_log_means(const float *raw, float *logd, int npix, int nviews, double *partials,
+void launch_log_means(const float *raw, float *logd, int nx, int ny, int nviews, double *partials,
                       float *means, unsigned *range, cudaStream_t st) {
   const dim3 grid(MEAN_CH, nviews);
-  if (logd) (range ? log_sum_kernel<true, true> : log_sum_kernel<true, false>)<<<grid, 256, 0, st>>>(raw, logd, npix, partials, range);
-  else (range ? log_sum_kernel<false, true> : log_sum_kernel<false, false>)<<<grid, 256, 0, st>>>(raw, nullptr, npix, partials, range);
+  const int npix = nx * ny;
+  if (logd) (range ? log_sum_kernel<true, true> : log_sum_kernel<true, false>)<<<grid, 256, 0, st>>>(raw, logd, npix, partials, nx, range);
+  else (range ? log_sum_kernel<false, true> : log_sum_kernel<false, false>)<<<grid, 256, 0, st>>>(raw, nullptr, npix, partials, nx, range);
   if (means) means_final_kernel<<<(nviews + 127) / 128, 128, 0, st>>>(partials, npix, nviews, means);
 }
 
@@ -301,19 +344,48 @@ template <int STORE> __device__ __forceinline__ void range_report(const FilterAr
 }
 
 // OCT staging, rows 2j and 2j+1 of element e: two of the element's eight halves in each
-// plane.  Infinities and NaN are noted in `top` (the largest magnitude bits of any
-// half): the tensor-core back-projector then leaves this block of rows to bp_oct_kernel.
+// plane.  The views' rows of a block of 8 share one scale, which the tensor cores' sums
+// over the views need.  A row whose own input is so far below the block's range that the
+// scale would leave it fewer bits than its transform has (the staging step 2^-25 against
+// 2^-27 of its largest sample) is staged with a scale of its own, and the tensor-core
+// kernel leaves its block to bp_oct_kernel; and so it does where a value is infinite or NaN
+// (`top`: the largest magnitude bits of any half).  The scale of its own leaves room for the
+// rounding that the row takes over from the row it shares its transform with (leak of that
+// one's range; a convolution takes none).  The line lies at gain * 2^-12 to 2^-13 of
+// the range (1/600 to 1/1300 at 2048 samples with the default cutoff): the intensities of rows
+// and views differ by less, an outlier (a hot pixel, a mask value) by more, and it costs only
+// its block.
+constexpr float OCT_LEAK = 0x1p-18f;  // the rounding of two transforms is below 2^-20 of the row pair's range
 struct OctWriter {
   uint32_t *out;     // this row pair's word of element 0 (elements are 4 words apart)
   size_t plane;      // words to the second plane
-  float scale;
+  float scale[2];
   uint32_t top = 0;
-  __device__ OctWriter(const FilterArgs &a, int v, int jp)
+  // warp_mx: the largest magnitudes of the two rows' input, by warp
+  __device__ OctWriter(const FilterArgs &a, int v, int jp, const uint2 *warp_mx, float leak)
       : out(reinterpret_cast<uint32_t *>(a.out) + (((size_t)v * a.rows_alloc + (jp >> 2)) * a.PW) * 4 + (jp & 3)),
-        plane((size_t)a.nviews * a.rows_alloc * a.PW * 4), scale(oct_scale(a.range, a.gain, false)) {}
+        plane((size_t)a.nviews * a.rows_alloc * a.PW * 4) {
+    const int blk = jp >> 2, nblk = (a.ny + 7) / 8;
+    uint2 m = make_uint2(0, 0);
+    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) m = make_uint2(max(m.x, warp_mx[w].x), max(m.y, warp_mx[w].y));
+    const float mx[2] = {__uint_as_float(m.x), __uint_as_float(m.y)};
+    const float least = fmaxf(mx[0], mx[1]) * leak;
+    const int common = oct_exponent(__uint_as_float(__ldg(&a.range[blk])), a.gain);
+    int p[2] = {common, common};
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+      if (mx[r] > 0.0f && __fmul_rn(mx[r], pow2f(common)) < 4.0f) {
+        p[r] = oct_exponent(fmaxf(mx[r], least), a.gain);
+        a.flags[blk] = a.flags[nblk] = 1;
+      }
+      scale[r] = pow2f(p[r]);
+    }
+    if (threadIdx.x == 0)
+      reinterpret_cast<char2 *>(a.exps)[((size_t)v * nblk + blk) * 4 + (jp & 3)] = make_char2((char)p[0], (char)p[1]);
+  }
   __device__ __forceinline__ void put(int e, float x0, float x1) {  // the samples of both rows
-    x0 = __fmul_rn(x0, scale);
-    x1 = __fmul_rn(x1, scale);
+    x0 = __fmul_rn(x0, scale[0]);
+    x1 = __fmul_rn(x1, scale[1]);
     const __half2 h = __floats2half2_rn(x0, x1);
     const uint32_t w = *reinterpret_cast<const uint32_t *>(&h);
     top = __vmaxu2(top, w & 0x7fff7fffu);
@@ -411,6 +483,8 @@ __device__ __forceinline__ void circulant_long(const float2 *A, float2 *B, const
 template <int FMT, int STORE>
 __global__ void __launch_bounds__(256) filter_kernel(FilterArgs a) {
   extern __shared__ __align__(16) unsigned char fsm[];
+  __shared__ uint2 warp_mx[FMT == FMT_OCT ? 8 : 1];
+  float mx0 = 0.0f, mx1 = 0.0f;
   const int n = a.nx;
   float2 *A = reinterpret_cast<float2 *>(fsm);
   float2 *B = A + n;
@@ -427,6 +501,14 @@ __global__ void __launch_bounds__(256) filter_kernel(FilterArgs a) {
       if (has1) x1 = __fsub_rn(x1, sb0[n + k]);
     }
     A[k] = make_float2(x0, x1);
+    if (FMT == FMT_OCT) {
+      mx0 = fmaxf(mx0, finite_abs(x0));
+      mx1 = fmaxf(mx1, finite_abs(x1));
+    }
+  }
+  if (FMT == FMT_OCT) {
+    const uint2 m = make_uint2(warp_max(mx0), warp_max(mx1));
+    if ((threadIdx.x & 31) == 0) warp_mx[threadIdx.x >> 5] = m;
   }
   __syncthreads();
   float2 *R = A;
@@ -486,7 +568,7 @@ __global__ void __launch_bounds__(256) filter_kernel(FilterArgs a) {
     return;
   }
   if (FMT == FMT_OCT) {  // each element is one sample
-    OctWriter ow(a, v, jp);
+    OctWriter ow(a, v, jp, warp_mx, a.conv_h ? 0.0f : OCT_LEAK);
     for (int e = threadIdx.x; e < a.PW; e += blockDim.x) {
       const int k = e - a.padL;
       float a0, a1 = 0.0f, b;
@@ -1002,6 +1084,17 @@ __device__ __forceinline__ void filter_p2_body(const FilterArgs &a, const int jp
     }
     x[j] = make_float2(x0, x1);
   }
+  __shared__ uint2 warp_mx[FMT == FMT_OCT ? T / 32 : 1];
+  if (FMT == FMT_OCT) {  // read behind the transforms' barriers
+    float mx0 = 0.0f, mx1 = 0.0f;
+#pragma unroll
+    for (int j = 0; j < V; ++j) {
+      mx0 = fmaxf(mx0, finite_abs(x[j].x));
+      mx1 = fmaxf(mx1, finite_abs(x[j].y));
+    }
+    const uint2 m = make_uint2(warp_max(mx0), warp_max(mx1));
+    if ((t & 31) == 0) warp_mx[t >> 5] = m;
+  }
   if (PAD) {
     __shared__ float2 part[T / 32];
     float2 s = make_float2(0.0f, 0.0f);
@@ -1072,7 +1165,7 @@ __device__ __forceinline__ void filter_p2_body(const FilterArgs &a, const int jp
   };
   float hmax = 0.0f;  // largest |value| packed into FP16 by this thread
   if constexpr (FMT == FMT_OCT) {  // each element is one sample
-    OctWriter ow(a, v, jp);
+    OctWriter ow(a, v, jp, warp_mx, OCT_LEAK);
     for (int e = t; e < a.PW; e += T) {
       const int k = e - a.padL;
       float2 z = k >= 0 && k < n ? fin(k) : fill(k);

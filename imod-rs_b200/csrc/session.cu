@@ -156,7 +156,7 @@ static void free_session(tg_session *s) {
   void *ptrs[] = {s->d_raw, s->d_logd, s->d_means, s->d_vol, s->d_sino, s->d_tmp, s->d_volg, s->d_volh, s->d_maxbits, s->d_mpart, s->d_pairs,
                   s->d_part, s->d_slice_stats, s->d_stats3, s->d_vg, s->d_vg2, s->d_weights,
                   s->d_conv, s->d_stretch, s->d_tw, s->d_err, s->d_lvinfo, s->d_lgoff, s->d_lxs,
-                  s->d_lys, s->d_lgdx, s->d_lgdy, s->d_ltab, s->d_xtb, s->d_lbnd, s->d_half, s->d_tmap, s->d_flags};
+                  s->d_lys, s->d_lgdx, s->d_lgdy, s->d_ltab, s->d_xtb, s->d_lbnd, s->d_half, s->d_tmap, s->d_oct};
   for (void *p : ptrs)
     if (p) cudaFree(p);
   for (auto &e : s->ev)
@@ -170,7 +170,7 @@ void free_session_async(tg_session *s, cudaStream_t after) {
   void *ptrs[] = {s->d_raw, s->d_logd, s->d_means, s->d_vol, s->d_sino, s->d_tmp, s->d_volg, s->d_volh, s->d_maxbits, s->d_mpart, s->d_pairs,
                   s->d_part, s->d_slice_stats, s->d_stats3, s->d_vg, s->d_vg2, s->d_weights,
                   s->d_conv, s->d_stretch, s->d_tw, s->d_err, s->d_lvinfo, s->d_lgoff, s->d_lxs,
-                  s->d_lys, s->d_lgdx, s->d_lgdy, s->d_ltab, s->d_xtb, s->d_lbnd, s->d_half, s->d_tmap, s->d_flags};
+                  s->d_lys, s->d_lgdx, s->d_lgdy, s->d_ltab, s->d_xtb, s->d_lbnd, s->d_half, s->d_tmap, s->d_oct};
   for (void *p : ptrs)
     if (p) cudaFreeAsync(p, after);
   for (auto &e : s->ev)
@@ -257,6 +257,12 @@ LocalDev local_dev(tg_session *s) {
   return L;
 }
 
+// d_oct: flags [blocks of 8 rows + 1], range [blocks], (8-byte aligned) exps [views][blocks][8]
+static size_t oct_blocks(const tg_session *s) { return (size_t)(s->ny + 7) / 8; }
+static size_t oct_bytes(const tg_session *s) { return (oct_blocks(s) + 1 + (size_t)s->nviews * oct_blocks(s)) * 8; }
+static unsigned *oct_range(const tg_session *s) { return reinterpret_cast<unsigned *>(s->d_oct) + oct_blocks(s) + 1; }
+static signed char *oct_exps(const tg_session *s) { return reinterpret_cast<signed char *>(oct_range(s) + oct_blocks(s) + 1); }
+
 BpArgs bp_args(tg_session *s, int mode) {
   BpArgs a{};
   a.pairs = s->d_pairs;
@@ -287,8 +293,11 @@ BpArgs bp_args(tg_session *s, int mode) {
   a.wait_limit_ns = s->wait_limit_ns;
   a.fault_skip_stage = s->fault_skip_stage;
   a.fill = !s->o.gpu_compat && s->o.fill_mode == TG_FILL_MEAN ? s->d_means : nullptr;
-  a.flags = s->d_flags;
-  a.range = reinterpret_cast<unsigned *>(s->d_err + 2);
+  if (s->mma_steps) {
+    a.flags = s->d_oct;
+    a.range = oct_range(s);
+    a.exps = oct_exps(s);
+  }
   a.gain = s->oct_gain;
   a.tmap = s->d_tmap;
   return a;
@@ -319,8 +328,11 @@ FilterArgs filter_args(tg_session *s, bool residual) {
   f.inv_n = 1.0f / (float)s->nx;
   f.plan = s->plan;
   f.err = s->d_err;
-  f.flags = s->d_flags;
-  f.range = reinterpret_cast<unsigned *>(s->d_err + 2);
+  if (s->mma_steps) {
+    f.flags = s->d_oct;
+    f.range = oct_range(s);
+    f.exps = oct_exps(s);
+  }
   f.gain = s->oct_gain;
   return f;
 }
@@ -430,24 +442,28 @@ FpArgs fp_args(tg_session *s) {
   return f;
 }
 
-// log10 and per-view means (main.rs:608-623).  On the tensor-core path FilterArgs::flags and
-// its range (d_err[2]) start over.
-static size_t oct_flags_bytes(const tg_session *s) { return ((size_t)(s->ny + 7) / 8 + 1) * 4; }
+// Before each staging on the tensor-core path: flags and ranges start over.
+static int oct_reset(tg_session *s) {
+  TG_CUDA(cudaMemsetAsync(s->d_oct, 0, (2 * oct_blocks(s) + 1) * 4, s->st));
+  return TG_OK;
+}
+
+// log10 and per-view means (main.rs:608-623)
 static int stage_log_means(tg_session *s) {
   if (s->mma_steps) {
-    TG_CUDA(cudaMemsetAsync(s->d_err + 2, 0, 4, s->st));
-    TG_CUDA(cudaMemsetAsync(s->d_flags, 0, oct_flags_bytes(s), s->st));
+    const int rc = oct_reset(s);
+    if (rc != TG_OK) return rc;
   }
-  launch_log_means(s->d_raw, s->d_logd, s->nx * s->ny, s->nz, s->d_mpart, s->means_pinned ? nullptr : s->d_means,
-                   s->mma_steps ? reinterpret_cast<unsigned *>(s->d_err + 2) : nullptr, s->st);
+  launch_log_means(s->d_raw, s->d_logd, s->nx, s->ny, s->nz, s->d_mpart, s->means_pinned ? nullptr : s->d_means,
+                   s->mma_steps ? oct_range(s) : nullptr, s->st);
   return TG_OK;
 }
 
 int stage_residual_range(tg_session *s, int *launches) {
   if (!s->mma_steps) return TG_OK;
-  unsigned *range = reinterpret_cast<unsigned *>(s->d_err + 2);
-  TG_CUDA(cudaMemsetAsync(range, 0, sizeof(unsigned), s->st));
-  launch_residual_range(s->d_logd ? s->d_logd : s->d_raw, s->d_sino, (size_t)s->nx * s->ny * s->nviews, range, s->st);
+  const int rc = oct_reset(s);
+  if (rc != TG_OK) return rc;
+  launch_residual_range(s->d_logd ? s->d_logd : s->d_raw, s->d_sino, s->nx, s->ny, s->nviews, oct_range(s), s->st);
   *launches += 1;
   return TG_OK;
 }
@@ -726,7 +742,7 @@ int tg::session_create_ex(const tg_geometry *g, const tg_options *opt, cudaMemPo
       (rc = dalloc(s, &s->d_tw, ((size_t)s->nx + std::max(s->nx, s->fft_n)) * 8)) ||
       (rc = dalloc(s, &s->d_stretch, (size_t)s->nviews * 4)) || (rc = dalloc(s, &s->d_err, 16)))
     return fail(rc);
-  if (s->mma_steps && ((rc = dalloc(s, &s->d_tmap, 128)) || (rc = dalloc(s, &s->d_flags, oct_flags_bytes(s)))))
+  if (s->mma_steps && ((rc = dalloc(s, &s->d_tmap, 128)) || (rc = dalloc(s, &s->d_oct, oct_bytes(s)))))
     return fail(rc);
   if (opt->log_transform && (rc = dalloc(s, &s->d_logd, nproj * 4))) return fail(rc);
   if (!opt->gpu_compat && opt->sirt_iters > 0 && (rc = dalloc(s, &s->d_sino, nproj * 4))) return fail(rc);
@@ -773,6 +789,7 @@ int tg::session_create_ex(const tg_geometry *g, const tg_options *opt, cudaMemPo
   // zero the staging buffer once: rows past ny stay zero
   if ((ce = cudaMemsetAsync(s->d_pairs, 0, s->pairs_bytes, s->st)) != cudaSuccess) return fail(cuda_fail(ce, "memset"));
   if ((ce = cudaMemsetAsync(s->d_err, 0, 16, s->st)) != cudaSuccess) return fail(cuda_fail(ce, "memset"));
+  if (s->d_oct && (ce = cudaMemsetAsync(s->d_oct, 0, oct_bytes(s), s->st)) != cudaSuccess) return fail(cuda_fail(ce, "memset"));
 
   std::vector<float> wt(s->nx);
   weight_table(s->nx, opt->radial_cutoff, opt->radial_falloff, opt->exact_filter_size, opt->hamming, wt.data());
@@ -1167,7 +1184,7 @@ int tg_session_view_sums(tg_session *s, double *sums) {
   TG_CUDA(cudaSetDevice(s->dev));
   double *d = nullptr;
   TG_CUDA(cudaMallocAsync((void **)&d, (size_t)s->nz * sizeof(double), s->st));
-  launch_log_means(s->d_raw, s->d_logd, s->nx * s->ny, s->nz, s->d_mpart, nullptr, nullptr, s->st);
+  launch_log_means(s->d_raw, s->d_logd, s->nx, s->ny, s->nz, s->d_mpart, nullptr, nullptr, s->st);
   launch_view_sums(s->d_mpart, s->nz, d, s->st);
   cudaError_t e = cudaGetLastError();
   if (e == cudaSuccess) e = cudaMemcpyAsync(sums, d, (size_t)s->nz * sizeof(double), cudaMemcpyDeviceToHost, s->st);

@@ -22,8 +22,8 @@ struct tg_session {  // one tilt series resident on a device
   int mma_steps = 0;       // fast or row-sum path on the tensor-core back-projector: its K steps (else 0)
   tg::TensorMap tmap{};    // TMA map of d_pairs on that path, and its copy for batched launches
   void *d_tmap = nullptr;
-  int *d_flags = nullptr;  // FilterArgs::flags on that path
-  float oct_gain = 1.0f;   // oct_scale's gain on that path
+  int *d_oct = nullptr;    // FilterArgs::flags, range and exps on that path
+  float oct_gain = 1.0f;   // oct_exponent's gain on that path
   float *xtb = nullptr;    // row sums (d_xtb, or the reprojector's FP32 copy, which is dead then)
   float *d_xtb = nullptr;
   int fp_fast = 0;  // reprojector: 0 general, 1 fast (no x-tilt), 2 fast with x-tilt

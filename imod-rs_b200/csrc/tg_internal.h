@@ -25,7 +25,7 @@ namespace tg {
 // FP32 float2 (a, b), FP16/BF16 uint32 h2(a, d).
 // OCT is FP32 staging for the tensor-core back-projector: 8 consecutive rows per
 // element, [plane][view][block of 8 rows][PW][8] halves; planes 0 and 1 hold the FP16
-// leading part and remainder of row[k] * oct_scale, k outside [0, nx) the edge sample's or 0
+// leading part and remainder of row[k] * 2^p (oct_exponent), k outside [0, nx) the edge sample's or 0
 // (a view's mean need not fit the rows' scale: the back-projector adds it itself, BpArgs::fill).
 enum Fmt { FMT_ROWPAIR = 0, FMT_SINGLE = 1, FMT_ROWS = 2 /* plain filtered rows, in place */, FMT_OCT = 3 };
 
@@ -42,29 +42,27 @@ struct StatPartial {
 
 // ---- log transform + per-view means (main.rs:608-623) ----
 // logd == nullptr: means of raw; else logd = log10(max(raw, 0.001)) and its means
-// (means == nullptr: partial sums only).  range (if given): raised to the largest finite
-// magnitude, as float bits
-void launch_log_means(const float *raw, float *logd, int npix, int nviews, double *partials,
+// (means == nullptr: partial sums only).  range (if given): raised, per block of 8 rows, to
+// the largest finite magnitude in any view, as float bits
+void launch_log_means(const float *raw, float *logd, int nx, int ny, int nviews, double *partials,
                       float *means, unsigned *range, cudaStream_t st);
-// the same of the residual in - sub of n values
-void launch_residual_range(const float *in, const float *sub, size_t n, unsigned *range, cudaStream_t st);
-// Power of two that the filtered rows of an OCT series are staged times: range is the
-// largest finite magnitude of the filter's input, gain a bound of the filter's amplification
-// (the 2-norm of the weights bounds the impulse response's 1-norm), so scaled rows stay
-// below 2^15; FP16 then holds 22 bits of every value down to 2^-17 of that bound.
-__host__ __device__ inline float oct_scale(const unsigned *range, float gain, bool inverse) {
-#ifdef __CUDA_ARCH__
-  const float m = fminf(__uint_as_float(*range) * gain, 1.0e38f);
-  if (!(m > 0.0f)) return 1.0f;
+// the same of the residual in - sub
+void launch_residual_range(const float *in, const float *sub, int nx, int ny, int nviews, unsigned *range, cudaStream_t st);
+#ifdef __CUDACC__
+// Exponent p of the power of two that filtered rows are staged times in OCT form: range is
+// the largest finite magnitude of the filter's input, gain a bound of the filter's
+// amplification (the 2-norm of the weights bounds the impulse response's 1-norm), so scaled
+// rows stay below 2^15.  FP16 then holds 22 bits of every value down to 2^-17 of that bound
+// and 2^-25 absolutely below.
+__device__ __forceinline__ int oct_exponent(float range, float gain) {
+  const float m = range * 0x1p-8f * gain;  // gain < 2^8: no overflow
+  if (!(m > 0.0f)) return 0;
   int e;
   frexpf(m, &e);  // m < 2^e
-  e = max(e, -100);
-  return ldexpf(1.0f, inverse ? e - 15 : 15 - e);
-#else
-  (void)range, (void)gain, (void)inverse;
-  return 1.0f;
-#endif
+  return min(15 - (e + 8), 126);
 }
+__device__ __forceinline__ float pow2f(int p) { return __int_as_float((127 + p) << 23); }  // -127 < p < 128
+#endif
 // per-view f64 sums from the partials of launch_log_means
 void launch_view_sums(const double *partials, int nviews, double *sums, cudaStream_t st);
 
@@ -96,8 +94,12 @@ struct FilterArgs {
   float inv_n;
   FftPlanDev plan;
   int *err;                 // session error word: bit 2 set when a value exceeds the FP16 range
-  int *flags;               // OCT, per block of 8 rows: 1 where a staged value is infinite or NaN; then 1 if any is
-  const unsigned *range;    // OCT: see oct_scale
+  // OCT, per block of 8 rows: its range in the filter's input (oct_exponent); flags: 1 where
+  // bp_oct_kernel takes the block (OctWriter), then 1 if it takes any; and the exponents
+  // of the rows, [view][block][8]
+  const unsigned *range;
+  int *flags;
+  signed char *exps;
   float gain;
 };
 void launch_filter(const FilterArgs &a, cudaStream_t st);
@@ -155,11 +157,12 @@ struct BpArgs {
   // stage of each tile, so the consumers' wait on it runs out; -1: none
   int fault_skip_stage;
   // tensor-core kernel: slices per tile (set by bp_mma_plan), and this pass's
-  // FilterArgs::flags, range and gain
+  // FilterArgs::flags, range, exps and gain
   int nper;
   const float *fill;        // mean mode: value of a view's samples outside its rows, else nullptr
   const int *flags;
   const unsigned *range;
+  const signed char *exps;
   const void *tmap;         // batched launches: the series' TensorMap, in device memory
   float gain;
   int pad_;
