@@ -254,6 +254,8 @@ int round_plan_launch_graph(RoundPlan &p, cudaStream_t st) {
 void round_plan_signature(const std::vector<tg_session *> &ss, std::vector<uint64_t> &key) {
   for (tg_session *s : ss) {
     key.push_back((uint64_t)s->variant);
+    key.push_back((uint64_t)s->fmt);  // these two change with the staging (tg_session_set_variant)
+    key.push_back((uint64_t)(uintptr_t)s->d_pairs);
     key.push_back((uint64_t)s->fp_variant);
   }
 }

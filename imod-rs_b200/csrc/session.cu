@@ -263,6 +263,21 @@ static size_t oct_bytes(const tg_session *s) { return (oct_blocks(s) + 1 + (size
 static unsigned *oct_range(const tg_session *s) { return reinterpret_cast<unsigned *>(s->d_oct) + oct_blocks(s) + 1; }
 static signed char *oct_exps(const tg_session *s) { return reinterpret_cast<signed char *>(oct_range(s) + oct_blocks(s) + 1); }
 
+// rows (row pairs, blocks of rows) that a view's staging holds
+static int staged_rows(int fmt, int ny) {
+  const int ra = bp_fast_row_align();  // a tile's row pairs never pass the allocation
+  return fmt == FMT_ROWPAIR ? ((ny + ra - 1) / ra) * (ra / 2) : fmt == FMT_OCT ? (ny + 15) / 16 * 2 : ny;
+}
+// the tensor map of a session's staging, for single launches and (d_tmap) batched ones
+static int write_tensor_map(tg_session *s) {
+  BpArgs a = bp_args(s, 0);
+  bp_mma_plan(a);
+  const int rc = bp_mma_tensor_map(s->d_pairs, s->nviews, s->rows_alloc, s->PW, a.nper, s->mma_steps, &s->tmap);
+  if (rc != TG_OK) return rc;
+  TG_CUDA(cudaMemcpyAsync(s->d_tmap, &s->tmap, sizeof s->tmap, cudaMemcpyHostToDevice, s->st));
+  return TG_OK;
+}
+
 BpArgs bp_args(tg_session *s, int mode) {
   BpArgs a{};
   a.pairs = s->d_pairs;
@@ -655,7 +670,7 @@ int tg::session_create_ex(const tg_geometry *g, const tg_options *opt, cudaMemPo
   if (const char *env = getenv("TG_BP_VARIANT")) oct = oct && atoi(env) == bp_fast_variants();  // fixed kernel
   else oct = oct && bp_mma_pays(s->onx, s->onz, s->ny, s->nviews);
   s->fmt = !s->fast && !s->xt_split ? FMT_SINGLE : oct ? FMT_OCT : FMT_ROWPAIR;
-  if (oct) s->mma_steps = bp_mma_steps(vg);
+  if (oct) s->mma_steps = s->oct_steps = bp_mma_steps(vg);
 
   // cosine stretch factors (main.rs:446-460); the reference indexes
   // tilt_angles[p] for every section p < nz and panics if the file is short.
@@ -695,10 +710,7 @@ int tg::session_create_ex(const tg_geometry *g, const tg_options *opt, cudaMemPo
     if (s->fmt == FMT_OCT) padR = std::max(padR, 32 - s->padL - s->nx);  // a whole staged window at least
     s->PW = (s->padL + s->nx + padR + 1) & ~1;
   }
-  const int ra = bp_fast_row_align();  // a tile's row pairs never pass the allocation
-  s->rows_alloc = s->fmt == FMT_ROWPAIR ? ((s->ny + ra - 1) / ra) * (ra / 2)
-                  : s->fmt == FMT_OCT   ? (s->ny + 15) / 16 * 2
-                                        : s->ny;
+  s->rows_alloc = staged_rows(s->fmt, s->ny);
 
   // transform of the register-resident filter kernel, else an FFT plan, else circulant.  A
   // reconstruction takes only the row's own length: a padded transform is nearer to 64 bits,
@@ -832,12 +844,7 @@ int tg::session_create_ex(const tg_geometry *g, const tg_options *opt, cudaMemPo
       (ce = cudaMemcpyAsync(s->d_vg2, vg2.data(), vg2.size() * 16, cudaMemcpyHostToDevice, s->st)) ||
       (ce = cudaMemcpyAsync(s->d_stretch, stretch.data(), stretch.size() * 4, cudaMemcpyHostToDevice, s->st)))
     return fail(cuda_fail(ce, "cudaMemcpy(setup)"));
-  if (s->mma_steps) {
-    BpArgs a = bp_args(s, 0);
-    bp_mma_plan(a);
-    if ((rc = bp_mma_tensor_map(s->d_pairs, s->nviews, s->rows_alloc, s->PW, a.nper, s->mma_steps, &s->tmap)) != TG_OK) return fail(rc);
-    if ((ce = cudaMemcpyAsync(s->d_tmap, &s->tmap, sizeof s->tmap, cudaMemcpyHostToDevice, s->st))) return fail(cuda_fail(ce, "cudaMemcpy(setup)"));
-  }
+  if (s->mma_steps && (rc = write_tensor_map(s)) != TG_OK) return fail(rc);
   if (!any_stretch) {
     if (pool) cudaFreeAsync(s->d_stretch, s->st);
     else cudaFree(s->d_stretch);
@@ -1206,6 +1213,39 @@ int tg_session_set_view_means(tg_session *s, const float *means) {
   return TG_OK;
 }
 
+// Moves a session that may run on the tensor cores to that kernel's staging or the fast
+// kernel's; the next run stages its rows anew.  On failure it stays as it was.
+static int restage(tg_session *s, bool mma) {
+  if (mma == (s->mma_steps != 0)) return TG_OK;
+  TG_CUDA(cudaSetDevice(s->dev));
+  TG_CUDA(cudaStreamSynchronize(s->st));
+  const int fmt = mma ? FMT_OCT : FMT_ROWPAIR, rows = staged_rows(fmt, s->ny);
+  const size_t bytes = (size_t)s->nviews * rows * s->PW * elem_bytes(fmt, s->store);
+  void *pairs = nullptr;
+  const int rc = dalloc(s, &pairs, bytes);
+  if (rc != TG_OK) return rc;
+  if (s->pool) TG_CUDA(cudaStreamSynchronize(s->own_st));  // the stream-ordered allocation exists
+  if (s->pool) cudaFreeAsync(s->d_pairs, s->own_st);
+  else cudaFree(s->d_pairs);
+  s->dev_bytes -= s->pairs_bytes;
+  s->d_pairs = pairs;
+  s->pairs_bytes = bytes;
+  s->fmt = fmt;
+  s->rows_alloc = rows;
+  s->mma_steps = mma ? s->oct_steps : 0;
+  if (s->sirt_exec) {  // captured iterations hold the old staging: capture again
+    cudaGraphExecDestroy(s->sirt_exec);
+    s->sirt_exec = nullptr;
+  }
+  TG_CUDA(cudaMemsetAsync(s->d_pairs, 0, bytes, s->st));  // rows past ny stay zero
+  if (mma) {
+    const int e = write_tensor_map(s);
+    if (e != TG_OK) return e;
+  }
+  TG_CUDA(cudaStreamSynchronize(s->st));
+  return TG_OK;
+}
+
 int tg_session_inject_wait_fault(tg_session *s, int32_t skip_stage, uint32_t wait_limit_us) {
   if (!s) return TG_ERR_INVALID_ARG;
   if (!s->fast && !s->xt_split) {
@@ -1224,8 +1264,13 @@ int tg_session_inject_wait_fault(tg_session *s, int32_t skip_stage, uint32_t wai
 }
 
 int tg_session_set_variant(tg_session *s, int32_t variant) {
-  if (!s || variant < -1 || variant >= bp_fast_variants() + (s->mma_steps ? 1 : 0)) return TG_ERR_INVALID_ARG;
-  if (!s->mma_steps) s->variant = variant;  // the tensor-core kernel has one tile shape
+  if (!s || variant < -1 || variant >= bp_fast_variants() + (s->oct_steps ? 1 : 0)) return TG_ERR_INVALID_ARG;
+  if (s->oct_steps) {  // a tile shape of the fast kernel, else (or by itself) the tensor cores
+    const bool mma = variant < 0 || variant == bp_fast_variants();
+    const int rc = restage(s, mma);
+    if (rc != TG_OK || mma) return rc;
+  }
+  s->variant = variant;
   return TG_OK;
 }
 

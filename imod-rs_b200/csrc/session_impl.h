@@ -20,6 +20,7 @@ struct tg_session {  // one tilt series resident on a device
   // views into xtb, then launch_xt_blend blends two rows per voxel into the volume
   bool xt_split = false;
   int mma_steps = 0;       // fast or row-sum path on the tensor-core back-projector: its K steps (else 0)
+  int oct_steps = 0;       // mma_steps of a series that takes that kernel by itself (set_variant may pin another)
   tg::TensorMap tmap{};    // TMA map of d_pairs on that path, and its copy for batched launches
   void *d_tmap = nullptr;
   int *d_oct = nullptr;    // FilterArgs::flags, range and exps on that path
