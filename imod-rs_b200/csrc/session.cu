@@ -667,7 +667,9 @@ int tg::session_create_ex(const tg_geometry *g, const tg_options *opt, cudaMemPo
   // FP32 staging of R-weighted rows back-projects on the tensor cores; without R-weighting the
   // result is the reference's bit for bit, which the fast kernel keeps.
   bool oct = (s->fast || s->xt_split) && s->store == TG_STORE_FP32 && !opt->no_weight;
-  if (const char *env = getenv("TG_BP_VARIANT")) oct = oct && atoi(env) == bp_fast_variants();  // fixed kernel
+  const char *env = getenv("TG_BP_VARIANT");  // fixed kernel, if it names one
+  const int pinned = env ? atoi(env) : -1;
+  if (pinned >= 0 && pinned <= bp_fast_variants()) oct = oct && pinned == bp_fast_variants();
   else oct = oct && bp_mma_pays(s->onx, s->onz, s->ny, s->nviews);
   s->fmt = !s->fast && !s->xt_split ? FMT_SINGLE : oct ? FMT_OCT : FMT_ROWPAIR;
   if (oct) s->mma_steps = s->oct_steps = bp_mma_steps(vg);

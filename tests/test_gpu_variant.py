@@ -71,6 +71,13 @@ def test_set_variant_between_batched_runs():
         b.close()
 
 
+@pytest.mark.parametrize("env,want", [("14", True), ("15", True), ("99", True), ("-1", True), ("0", False), ("13", False)])
+def test_environment_names_a_kernel_or_is_ignored(env, want, monkeypatch):
+    monkeypatch.setenv("TG_BP_VARIANT", env)
+    with make() as s:
+        assert tensor(s) == want
+
+
 def test_what_is_no_variant_is_refused():
     with make() as s, make(storage="fp16") as h:
         for v in (-2, 15):
