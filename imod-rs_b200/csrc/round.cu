@@ -186,10 +186,7 @@ int round_plan_issue(RoundPlan &p, cudaStream_t st) {
                                        reinterpret_cast<const int *>(d + g.fpb), g.nfp, st);
   for (tg_session *s : p.fp_single) launches += launch_reproject(fp_args(s), st);
   for (tg_session *s : p.scaled) {
-    const cudaStream_t own = s->st;
-    s->st = st;
-    const int rc = stage_residual_range(s, &launches);
-    s->st = own;
+    const int rc = stage_residual_range(s, st, &launches);
     if (rc != TG_OK) return rc;
   }
   for (const RoundPlan::Fi &g : p.fi) {

@@ -458,15 +458,15 @@ FpArgs fp_args(tg_session *s) {
 }
 
 // Before each staging on the tensor-core path: flags and ranges start over.
-static int oct_reset(tg_session *s) {
-  TG_CUDA(cudaMemsetAsync(s->d_oct, 0, (2 * oct_blocks(s) + 1) * 4, s->st));
+static int oct_reset(tg_session *s, cudaStream_t st) {
+  TG_CUDA(cudaMemsetAsync(s->d_oct, 0, (2 * oct_blocks(s) + 1) * 4, st));
   return TG_OK;
 }
 
 // log10 and per-view means (main.rs:608-623)
 static int stage_log_means(tg_session *s) {
   if (s->mma_steps) {
-    const int rc = oct_reset(s);
+    const int rc = oct_reset(s, s->st);
     if (rc != TG_OK) return rc;
   }
   launch_log_means(s->d_raw, s->d_logd, s->nx, s->ny, s->nz, s->d_mpart, s->means_pinned ? nullptr : s->d_means,
@@ -474,11 +474,11 @@ static int stage_log_means(tg_session *s) {
   return TG_OK;
 }
 
-int stage_residual_range(tg_session *s, int *launches) {
+int stage_residual_range(tg_session *s, cudaStream_t st, int *launches) {
   if (!s->mma_steps) return TG_OK;
-  const int rc = oct_reset(s);
+  const int rc = oct_reset(s, st);
   if (rc != TG_OK) return rc;
-  launch_residual_range(s->d_logd ? s->d_logd : s->d_raw, s->d_sino, s->nx, s->ny, s->nviews, oct_range(s), s->st);
+  launch_residual_range(s->d_logd ? s->d_logd : s->d_raw, s->d_sino, s->nx, s->ny, s->nviews, oct_range(s), st);
   *launches += 1;
   return TG_OK;
 }
@@ -890,7 +890,7 @@ namespace tg {
 int sirt_iterations(tg_session *s, int n) {
   auto one_iter = [&]() -> int {
     s->iter_launches = launch_reproject(fp_args(s), s->st) + 1 + bp_launch_count(s);
-    const int rc = stage_residual_range(s, &s->iter_launches);
+    const int rc = stage_residual_range(s, s->st, &s->iter_launches);
     if (rc != TG_OK) return rc;
     launch_filter(filter_args(s, true), s->st);
     return launch_bp(s, 2, nullptr);

@@ -112,7 +112,7 @@ int autotune(tg_session *s);
 // the tile variant already tuned for this shape (or pinned by TG_BP_VARIANT), else -1
 int tune_lookup(tg_session *s);
 // before the filter of a SIRT residual on the tensor-core path: the residual's range
-int stage_residual_range(tg_session *s, int *launches);
+int stage_residual_range(tg_session *s, cudaStream_t st, int *launches);
 // log10 + per-view means, then the filter stage of the WBP pass
 int stage_front(tg_session *s, int *launches);
 // fake-SIRT passes, output transform (when the volume was stored raw) and statistics;
