@@ -16,7 +16,6 @@
 #include <sys/mman.h>
 
 #include <algorithm>
-#include <system_error>
 #include <thread>
 
 #ifndef MADV_POPULATE_WRITE
@@ -50,7 +49,7 @@ class FaultAhead {
               return;
         });
         ++n_;
-      } catch (const std::system_error &) {  // no more threads: the copy faults the rest in
+      } catch (...) {  // no thread or no memory for one: the copy faults the rest in
         break;
       }
     }
