@@ -24,8 +24,9 @@
 //   rows out    inverse FFT -> real part, scaled
 //   combine     per pixel, the strips that hold it, in strip order
 // Each CTA transforms several rows at once, so the transposed stores cover
-// whole 32-byte sectors.  A chunk's strips stay in L2 (CTF_CHUNK_BYTES), and
-// the copy of the next chunk's views overlaps the kernels of this one.
+// whole 32-byte sectors.  A chunk's strips stay in L2 (CTF_CHUNK_BYTES).  Copies
+// and kernels share one stream: while a chunk's kernels run, the host only stages
+// the next chunk's pageable views.
 // 512x512x41 with 16-pixel strips (1312 strips), host to host: 88.7 ms with nine
 // launches per strip (11,852 launches, bound by the launching thread and by
 // grids of a few blocks), 18.0 ms batched, of which the copies from and to the

@@ -74,7 +74,9 @@ def reconstruct_slab(proj_slab, angles, nx: int, ny_total: int, sum_views=all_re
     add the per-view sums over the ranks (sum_views), pin the whole series' mean fill
     values, reconstruct.  Returns the slab's volume and its per-slice statistics.
     Not for x-tilt, local alignment or fake SIRT (their rows or slices reach across
-    slab edges)."""
+    slab edges).  A slab of few rows may take another FP32 back-projector than the whole
+    series (equal to about 1e-7); with TG_BP_VARIANT set alike, slabs and whole agree in
+    every bit."""
     import tiltgpu as T
 
     nz, ny, _ = proj_slab.shape
