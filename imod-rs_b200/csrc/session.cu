@@ -716,7 +716,7 @@ int tg::session_create_ex(const tg_geometry *g, const tg_options *opt, cudaMemPo
 
   // transform of the register-resident filter kernel, else an FFT plan, else circulant.  A
   // reconstruction takes only the row's own length: a padded transform is nearer to 64 bits,
-  // but it moves a volume's mean, a small difference of large sums, by up to 1e-2 of itself
+  // but it moves a volume's mean, a small difference of large sums, by up to 7e-2 of itself
   // and, in half staging, every rounding decision near a midpoint.
   s->fft_n = opt->no_weight || getenv("TG_FILTER_GENERIC") ? 0 : p2_transform_length(s->nx);
   if (!rows_only && s->fft_n != s->nx) s->fft_n = 0;
