@@ -36,6 +36,7 @@ class FaultAhead {
     }
     if (at.type != cudaMemoryTypeUnregistered) return;
     const uintptr_t lo = ((uintptr_t)host + PAGE - 1) / PAGE * PAGE, hi = ((uintptr_t)host + bytes) / PAGE * PAGE;
+    if (present(lo, hi)) return;
     const uintptr_t share = ((hi - lo) / THREADS + BLOCK - 1) / BLOCK * BLOCK;
     for (int i = 0; i < THREADS; ++i) {
       const uintptr_t a = lo + i * share, b = std::min(hi, a + share);
@@ -62,7 +63,17 @@ class FaultAhead {
   }
 
  private:
-  static constexpr int THREADS = 4;
+  // A buffer that was filled before has its pages; a few tell, and starting the threads for
+  // nothing would cost a small download several percent.
+  static bool present(uintptr_t lo, uintptr_t hi) {
+    for (int i = 0; i < PROBES; ++i) {
+      const uintptr_t page = (lo + (hi - PAGE - lo) / (PROBES - 1) * i) / PAGE * PAGE;
+      unsigned char in = 0;
+      if (mincore(reinterpret_cast<void *>(page), PAGE, &in) != 0 || !(in & 1)) return false;
+    }
+    return true;
+  }
+  static constexpr int THREADS = 4, PROBES = 16;
   static constexpr uintptr_t PAGE = 4096, BLOCK = 2u << 20;
   static constexpr size_t MIN_BYTES = 4u << 20;
   std::thread th_[THREADS];
