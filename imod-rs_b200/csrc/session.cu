@@ -268,14 +268,10 @@ static int staged_rows(int fmt, int ny) {
   const int ra = bp_fast_row_align();  // a tile's row pairs never pass the allocation
   return fmt == FMT_ROWPAIR ? ((ny + ra - 1) / ra) * (ra / 2) : fmt == FMT_OCT ? (ny + 15) / 16 * 2 : ny;
 }
-// the tensor map of a session's staging, for single launches and (d_tmap) batched ones
-static int write_tensor_map(tg_session *s) {
+static int make_tensor_map(tg_session *s, void *pairs, int rows, int steps, TensorMap *map) {
   BpArgs a = bp_args(s, 0);
   bp_mma_plan(a);
-  const int rc = bp_mma_tensor_map(s->d_pairs, s->nviews, s->rows_alloc, s->PW, a.nper, s->mma_steps, &s->tmap);
-  if (rc != TG_OK) return rc;
-  TG_CUDA(cudaMemcpyAsync(s->d_tmap, &s->tmap, sizeof s->tmap, cudaMemcpyHostToDevice, s->st));
-  return TG_OK;
+  return bp_mma_tensor_map(pairs, s->nviews, rows, s->PW, a.nper, steps, map);
 }
 
 BpArgs bp_args(tg_session *s, int mode) {
@@ -846,7 +842,11 @@ int tg::session_create_ex(const tg_geometry *g, const tg_options *opt, cudaMemPo
       (ce = cudaMemcpyAsync(s->d_vg2, vg2.data(), vg2.size() * 16, cudaMemcpyHostToDevice, s->st)) ||
       (ce = cudaMemcpyAsync(s->d_stretch, stretch.data(), stretch.size() * 4, cudaMemcpyHostToDevice, s->st)))
     return fail(cuda_fail(ce, "cudaMemcpy(setup)"));
-  if (s->mma_steps && (rc = write_tensor_map(s)) != TG_OK) return fail(rc);
+  if (s->mma_steps) {  // for single launches and (d_tmap) batched ones
+    if ((rc = make_tensor_map(s, s->d_pairs, s->rows_alloc, s->mma_steps, &s->tmap)) != TG_OK) return fail(rc);
+    if ((ce = cudaMemcpyAsync(s->d_tmap, &s->tmap, sizeof s->tmap, cudaMemcpyHostToDevice, s->st)))
+      return fail(cuda_fail(ce, "cudaMemcpy(setup)"));
+  }
   if (!any_stretch) {
     if (pool) cudaFreeAsync(s->d_stretch, s->st);
     else cudaFree(s->d_stretch);
@@ -1226,9 +1226,18 @@ static int restage(tg_session *s, bool mma) {
   void *pairs = nullptr;
   const int rc = dalloc(s, &pairs, bytes);
   if (rc != TG_OK) return rc;
-  if (s->pool) TG_CUDA(cudaStreamSynchronize(s->own_st));  // the stream-ordered allocation exists
-  if (s->pool) cudaFreeAsync(s->d_pairs, s->own_st);
-  else cudaFree(s->d_pairs);
+  auto release = [&](void *p) { return s->pool ? cudaFreeAsync(p, s->own_st) : cudaFree(p); };
+  cudaError_t ce = s->pool ? cudaStreamSynchronize(s->own_st) : cudaSuccess;  // the stream-ordered allocation exists
+  if (ce == cudaSuccess) ce = cudaMemsetAsync(pairs, 0, bytes, s->st);  // rows past ny stay zero
+  int err = ce == cudaSuccess ? TG_OK : cuda_fail(ce, "staging buffer");
+  TensorMap map{};
+  if (err == TG_OK && mma) err = make_tensor_map(s, pairs, rows, s->oct_steps, &map);
+  if (err != TG_OK) {
+    release(pairs);
+    s->dev_bytes -= bytes;
+    return err;
+  }
+  release(s->d_pairs);
   s->dev_bytes -= s->pairs_bytes;
   s->d_pairs = pairs;
   s->pairs_bytes = bytes;
@@ -1239,10 +1248,9 @@ static int restage(tg_session *s, bool mma) {
     cudaGraphExecDestroy(s->sirt_exec);
     s->sirt_exec = nullptr;
   }
-  TG_CUDA(cudaMemsetAsync(s->d_pairs, 0, bytes, s->st));  // rows past ny stay zero
   if (mma) {
-    const int e = write_tensor_map(s);
-    if (e != TG_OK) return e;
+    s->tmap = map;
+    TG_CUDA(cudaMemcpyAsync(s->d_tmap, &s->tmap, sizeof s->tmap, cudaMemcpyHostToDevice, s->st));
   }
   TG_CUDA(cudaStreamSynchronize(s->st));
   return TG_OK;
