@@ -55,11 +55,12 @@ void launch_residual_range(const float *in, const float *sub, int nx, int ny, in
 // rows stay below 2^15.  FP16 then holds 22 bits of every value down to 2^-17 of that bound
 // and 2^-25 absolutely below.
 __device__ __forceinline__ int oct_exponent(float range, float gain) {
-  const float m = range * 0x1p-8f * gain;  // gain < 2^8: no overflow
+  const bool large = range > 1.0f;
+  const float m = (large ? range * 0x1p-8f : range) * gain;  // 1 <= gain < 2^8: no overflow, no underflow
   if (!(m > 0.0f)) return 0;
   int e;
   frexpf(m, &e);  // m < 2^e
-  return min(15 - (e + 8), 126);
+  return min(15 - (large ? e + 8 : e), 126);
 }
 __device__ __forceinline__ float pow2f(int p) { return __int_as_float((127 + p) << 23); }  // -127 < p < 128
 #endif

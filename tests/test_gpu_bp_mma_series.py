@@ -294,3 +294,18 @@ def test_views_of_many_magnitudes(monkeypatch):
         assert rel_l2(got, want) <= TOL
         alone = np.abs(want) <= 20 * faint
         assert alone.any() and rel_l2(got[alone], want[alone]) <= TOL
+
+
+@pytest.mark.parametrize("e", [-126, -118, -60, 100, 112])
+def test_data_near_the_ends_of_the_f32_range(e, monkeypatch):
+    ang = angles(-60, 60, 12)
+    proj = np.ldexp(smooth_stack(len(ang), 20, 64, seed=8), e).astype(np.float32)
+
+    def run():
+        with session(64, 20, ang, proj, thickness=24) as s:
+            s.reconstruct()
+            return s.download()[0]
+    want, got = both(monkeypatch, run)
+    # results below the smallest normal number are rounded to its 2^-23
+    tiny = 2.0 ** -148 * np.sqrt(want.size)
+    assert np.linalg.norm(np.ldexp(got.astype(np.float64) - want, 100)) <= np.ldexp(TOL * np.linalg.norm(want.astype(np.float64)) + tiny, 100)
